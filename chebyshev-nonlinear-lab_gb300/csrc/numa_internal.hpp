@@ -361,6 +361,7 @@ private:
 };
 
 // ------------------------------------------------------------------------------ PoissonMG
+struct CoarseParams;
 class PoissonMG {
 public:
     PoissonMG(Context& ctx, size_t n, int pre, int post, int precision, int max_levels);
@@ -398,6 +399,11 @@ private:
     size_t tail_l_ = SIZE_MAX;
     size_t tail_smem_ = 0;
     void launch_tail32();
+    // FP64 cycle: the levels from cl_l_ down run in one kernel (mg_coarse.cuh); SIZE_MAX = none.
+    size_t cl_l_ = SIZE_MAX;
+    size_t coarse_params(size_t l, CoarseParams& cp) const;
+    void plan_coarse();
+    void launch_coarse(const double* b, double* x);
     // The levels below the finest touch only the hierarchy's own arrays, so their part of the
     // cycle is captured once into a CUDA graph and replayed (one launch instead of ~10 a level).
     void coarse_cycle();

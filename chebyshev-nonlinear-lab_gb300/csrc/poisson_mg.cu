@@ -24,7 +24,7 @@
 #include <limits>
 #include <type_traits>
 
-#include "mg_kernels.cuh"
+#include "mg_coarse.cuh"
 
 namespace numa::gpu {
 
@@ -79,14 +79,7 @@ PoissonMG::PoissonMG(Context& ctx, size_t n, int pre, int post, int precision, i
         L->h2inv = h2;
         L->inv = 1.0 / h2;
         const size_t Nl = m * m * m;
-        const bool finest = levels_.empty();
-        if (precision == NUMA_GPU_FP64) {
-            L->bs64.resize(Nl);
-            if (!finest) {
-                L->x64.resize(Nl);
-                L->b64.resize(Nl);
-            }
-        } else {
+        if (precision == NUMA_GPU_FP32) {
             // x is padded by more than one plane of a colour on both sides, b and b h^2 at the end:
             // the FP32 kernels load every neighbour unconditionally (boundary values are then
             // replaced by zero with a select), and no load leaves the allocation
@@ -102,8 +95,20 @@ PoissonMG::PoissonMG(Context& ctx, size_t n, int pre, int post, int precision, i
         m = (m - 1) / 2;
         h2 /= 4.0;
     }
+    if (precision == NUMA_GPU_FP64) {
+        plan_coarse();
+        for (size_t l = 0; l < levels_.size() && l <= cl_l_; ++l) {  // below, the levels live in shared memory
+            Level& L = *levels_[l];
+            const size_t Nl = (size_t)L.n * L.n * L.n;
+            L.bs64.resize(Nl);
+            if (l > 0) {
+                L.x64.resize(Nl);
+                L.b64.resize(Nl);
+            }
+        }
+    }
     if (levels_.size() > 1) {
-        if (precision == NUMA_GPU_FP64) scratch_r_.resize(N0_);
+        if (precision == NUMA_GPU_FP64) scratch_r_.resize(cl_l_ > 0 ? N0_ : 0);
         else scratch_r_.resize((N0_ + 1) / 2);  // N0 floats
     }
     // FP32: the levels of n <= 15 below the finest run as one CTA with shared-memory arrays
@@ -150,11 +155,83 @@ void PoissonMG::launch_tail32() {
     ctx_.check_launch("mg tail (fp32)");
 }
 
+namespace {
+
+cudaLaunchConfig_t coarse_config(cudaLaunchAttribute (&attr)[2], int cluster, size_t smem, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cluster);
+    cfg.blockDim = dim3(kCoarseThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cfg;
+}
+
+}  // namespace
+
+// The coarse kernel's parameters for the FP64 cycle from level l down; returns its shared memory in bytes.
+size_t PoissonMG::coarse_params(size_t l, CoarseParams& cp) const {
+    int n[kCoarseMax];
+    double h2[kCoarseMax];
+    for (size_t m = l; m < levels_.size(); ++m) {
+        n[m - l] = levels_[m]->n;
+        h2[m - l] = levels_[m]->h2inv;
+    }
+    cp = CoarseParams{};
+    cp.pre = pre_;
+    cp.post = post_;
+    return coarse_layout(cp, n, h2, (int)(levels_.size() - l));
+}
+
+// Where the coarse kernel takes over (mg_coarse.cuh): the first level of n <= kCoarseTop whose cycle fits the
+// shared memory of a cluster the device can schedule.
+void PoissonMG::plan_coarse() {
+    for (size_t l = 0; l < levels_.size(); ++l) {
+        if (levels_[l]->n > kCoarseTop || levels_.size() - l > (size_t)kCoarseMax) continue;
+        CoarseParams cp;
+        const size_t bytes = coarse_params(l, cp);
+        if (bytes > (size_t)set_dynamic_smem_limit(ctx_, k_mg_coarse)) continue;
+        if (cp.cluster > 1) {
+            cudaLaunchAttribute attr[2];
+            const cudaLaunchConfig_t cfg = coarse_config(attr, cp.cluster, bytes, ctx_.stream);
+            int clusters = 0;
+            const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, k_mg_coarse, &cfg);
+            if (e != cudaSuccess || clusters < 1) {
+                cudaGetLastError();
+                continue;
+            }
+        }
+        cl_l_ = l;
+        return;
+    }
+}
+
+// x = the FP64 cycle from level cl_l_ down applied to b.
+void PoissonMG::launch_coarse(const double* b, double* x) {
+    CoarseParams cp;
+    const size_t bytes = coarse_params(cl_l_, cp);
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = coarse_config(attr, cp.cluster, bytes, ctx_.stream);
+    NUMA_CUDA(cudaLaunchKernelEx(&cfg, k_mg_coarse, cp, b, x));
+    ctx_.count_launch();
+    ctx_.check_launch("mg coarse levels");
+}
+
 PoissonMG::~PoissonMG() {
     if (coarse_exec_) cudaGraphExecDestroy(coarse_exec_);
 }
 
 void PoissonMG::coarse_cycle() {
+    if (cl_l_ == 1) {  // one kernel: no graph
+        launch_coarse(levels_[1]->b64.p, levels_[1]->x64.p);
+        return;
+    }
     if (coarse_exec_ && graph_jac_ != coarse_jac_) {  // captured in the other tail mode
         cudaGraphExecDestroy(coarse_exec_);
         coarse_exec_ = nullptr;
@@ -189,6 +266,10 @@ void PoissonMG::coarse_cycle() {
 template <class T>
 void PoissonMG::cycle(size_t l) {
     Level& L = *levels_[l];
+    if (l == cl_l_) {
+        launch_coarse(L.b64.p, L.x64.p);
+        return;
+    }
     const int n = L.n;
     const bool finest = (l == 0);
     T* x = finest ? static_cast<T*>(x0_) : xp<T>(L);
@@ -413,6 +494,10 @@ void PoissonMG::apply(const double* r, double* z) {
     Level& L0 = *levels_[0];
     const size_t N = N0_;
     if (precision_ == NUMA_GPU_FP64) {
+        if (cl_l_ == 0) {  // (r and z may be the same vector)
+            launch_coarse(r, z);
+            return;
+        }
         const double* b = r;
         if (r == z) {
             alias_b_.resize(N);
