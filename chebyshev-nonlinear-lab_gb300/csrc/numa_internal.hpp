@@ -432,18 +432,25 @@ private:
 // 2D V-cycle for alpha I - nu Lap_h (linalg/helmholtz_mg2d.hpp:13-158), FP64, bit-exact.
 class HelmholtzMG2D {
 public:
-    HelmholtzMG2D(Context& ctx, size_t n, double alpha, double nu, int pre, int post);
+    // fields: vectors of n^2 values cycled together (u and v of Burgers2D), one after the other in r and z
+    HelmholtzMG2D(Context& ctx, size_t n, double alpha, double nu, int pre, int post, int fields = 1);
     ~HelmholtzMG2D();
     size_t levels() const { return levels_.size(); }
     size_t size() const { return N0_; }
-    // z = V-cycle(r), n^2 FP64 device vectors (helmholtz_mg2d.hpp:36-42).
+    // z = V-cycle(r), fields of n^2 FP64 values (helmholtz_mg2d.hpp:36-42).
     void apply(const double* r, double* z);
     struct Level;
 
 private:
     void cycle(size_t l);
+    void launch_tail(const double* b, double* x);
+    void coarse_cycle();
     Context& ctx_;
     size_t N0_;
+    int fields_;
+    size_t tail_l_ = SIZE_MAX;  // the levels from here down run in one CTA a field
+    cudaGraphExec_t exec_ = nullptr;
+    uint64_t graph_kernels_ = 0;
     double alpha_;
     int pre_, post_;
     std::vector<std::unique_ptr<Level>> levels_;
