@@ -60,6 +60,27 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// Warp-wide sums of R values per lane (R a power of two up to 32): afterwards v[0] of every lane is the sum of
+// value lane >> (5 - log2 R).  Each step adds half of the values a lane still holds to its partner's, so the
+// warp issues about R FP64 additions instead of the 5 R of R separate butterflies: an FP64 warp instruction
+// occupies the SM's pipe for 16 cycles, and sixteen butterflies on eight warps would take 10,000.
+template <int R>
+__device__ __forceinline__ void warp_sum_scatter(double (&v)[R]) {
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int n = R; n > 1; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int k = 0; k < n / 2; ++k) {
+            const double send = up ? v[k] : v[k + n / 2], keep = up ? v[k + n / 2] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+}
+
 // Block-wide sum of R values per thread; every thread of the block must call it.  Returns the
 // block totals in warp 0 lane 0 (others hold unspecified values).
 template <int R>

@@ -9,6 +9,17 @@
 //  * MGS (reference, gmres.hpp:141-144): one kernel per basis vector, each fusing the previous
 //    axpy w -= h_{i-1} V_{i-1} (one FMA) with the next inner product <w, V_i>; the last one fuses
 //    the final axpy with ||w||.  2(j+1)+1 FP64 operations per point, j+2 launches per step.
+//  * MGS with more than kIcwyFrom basis vectors, up to kIcwyMax, of at most kIcwyMaxN points: the inverse compact
+//    WY form (K. Swirydowicz, J. Langou, S. Ananthan, U. Yang, S. Thomas, "Low synchronization Gram-Schmidt and
+//    generalized minimal residual algorithms", Numer. Linear Algebra Appl. 28(2), 2021).  MGS's coefficients
+//    h_i = <w - sum_{l<i} h_l V_l, V_i> solve (I + L) h = V^T w with L the strictly lower part of V^T V, so one
+//    kernel takes all inner products of w and of the newest V_j with the basis (the new row of L) and its last
+//    block substitutes forward; the second subtracts h_i V_i in MGS's order and takes the norm.  The loss of
+//    orthogonality is MGS's, O(eps kappa).  Two reductions a step instead of j + 2, which is what bounds the
+//    chain on short vectors (~5 us each), for 3(j+1) FP64 operations per point, which is what bounds both on
+//    long ones.  A whole GMRES step (unpreconditioned, restart 30 / 8 / 2), chain against compact form
+//    throughout: 31^3 115 / 58 / 57 us against 46 / 47 / 62; 95^3 261 / 133 / 136 against 186 / 126 / 162;
+//    127^3 351 / 187 / 197 against 338 / 208 / 250: hence both limits.
 //  * CGS2: h = V^T w; w -= V h fused with h' = V^T w; w -= V h' fused with ||w||; H = h + h'.
 //    Three passes over the basis, 4(j+1)+1 FP64 operations per point.
 //  * CGS1: h = V^T w; w -= V h fused with ||w|| (2j + 5 vector passes).
@@ -60,6 +71,159 @@ __global__ void __launch_bounds__(kRedThreads) k_mgs(double* __restrict__ w, con
     }
     block_sum<1>(s, sm);
     grid_reduce_finish<1>(s, red, fin);
+}
+
+// ---- modified Gram-Schmidt in the inverse compact WY form (see the head of the file)
+constexpr int kIcwyFrom = 4;               // the first kIcwyFrom vectors of a cycle go through the chain
+constexpr int kIcwyMax = 32;               // basis vectors: the last block's warp substitutes, a lane a vector
+constexpr size_t kIcwyMaxN = 1 << 20;
+constexpr int kIcwyRow = kIcwyMax + 1;     // row stride of L in shared memory
+static_assert(kIcwyMax / 8 * 16 <= kMaxRedResults, "partial sums of the inner products");
+
+// hcol[0..j] = h of MGS for w against V_0 .. V_j, and row j of gram (kIcwyMax wide) = <V_j, V_i>, i < j.
+// blockIdx.y takes eight vectors; results 16 y + r (<w, V_{8y+r}>) and 16 y + 8 + r (<V_j, V_{8y+r}>).
+// START (j = kIcwyFrom): the last blockIdx.y takes the rows of L that the chain's steps left out, <V_a, V_b> for
+// b < a < kIcwyFrom, as its results a (a - 1) / 2 + b.
+template <bool START>
+__global__ void __launch_bounds__(kRedThreads) k_icwy_dots(const double* __restrict__ w, const double* __restrict__ V,
+                                                           size_t N, int j, RedArgs red, double* __restrict__ gram,
+                                                           double* __restrict__ hcol) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ double sm[kRedThreads / 32][16];
+    __shared__ double res[kIcwyMax / 8 * 16];
+    __shared__ double L[kIcwyMax * kIcwyRow];
+    __shared__ bool am_last;
+    const bool start = START && blockIdx.y == gridDim.y - 1;
+    const int i0 = start ? 0 : blockIdx.y * 8, cnt = start ? kIcwyFrom : min(8, j + 1 - i0), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const double* vj = V + (size_t)j * N;
+    const double* Vb = V + (size_t)i0 * N;
+    double a[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) a[r] = 0.0;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+#pragma unroll 2
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + tid; i < N; i += stride) {
+        const double wi = w[i], vji = vj[i];
+        double v[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) v[r] = r < cnt ? Vb[(size_t)r * N + i] : 0.0;
+        if (START && start) {
+#pragma unroll
+            for (int p = 1; p < kIcwyFrom; ++p)
+#pragma unroll
+                for (int q = 0; q < p; ++q) a[p * (p - 1) / 2 + q] = __fma_rn(v[p], v[q], a[p * (p - 1) / 2 + q]);
+            continue;
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            if (r < cnt) a[r] = __fma_rn(wi, v[r], a[r]);
+            if (i0 + r < j) a[8 + r] = __fma_rn(vji, v[r], a[8 + r]);
+        }
+    }
+    warp_sum_scatter<16>(a);
+    if (!(lane & 1)) sm[warp][lane >> 1] = a[0];
+    __syncthreads();
+    if (tid < 128) {
+        double s = sm[tid & 7][tid >> 3];
+        s += __shfl_xor_sync(0xffffffffu, s, 4);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        if (!(tid & 7)) {
+            red.partials[(size_t)(blockIdx.y * 16 + (tid >> 3)) * kMaxRedBlocks + blockIdx.x] = s;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    if (tid == 0) am_last = atomicAdd(red.ticket, 1u) == gridDim.x * gridDim.y - 1;
+    __syncthreads();
+    if (!am_last) return;
+    __threadfence();
+    for (int t = tid; !START && t < j * kIcwyMax; t += kRedThreads)
+        L[(t / kIcwyMax) * kIcwyRow + t % kIcwyMax] = gram[t];
+    if (warp < (int)gridDim.y) {
+        double s[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) s[r] = 0.0;
+        for (unsigned b = lane; b < gridDim.x; b += 32) {
+#pragma unroll
+            for (int r = 0; r < 16; ++r) s[r] += __ldcg(red.partials + (size_t)(warp * 16 + r) * kMaxRedBlocks + b);
+        }
+        warp_sum_scatter<16>(s);
+        if (!(lane & 1)) res[warp * 16 + (lane >> 1)] = s[0];
+    }
+    __syncthreads();
+    if (START && tid < kIcwyFrom * kIcwyFrom) {
+        const int p = tid / kIcwyFrom, q = tid % kIcwyFrom;
+        if (q < p) {
+            const double l = res[(gridDim.y - 1) * 16 + p * (p - 1) / 2 + q];
+            L[p * kIcwyRow + q] = l;
+            gram[p * kIcwyMax + q] = l;
+        }
+    }
+    if (START) __syncthreads();
+    if (warp == 0) {
+        const auto at = [&](int i, int off) { return res[(i >> 3) * 16 + off + (i & 7)]; };
+        if (lane < j) {
+            const double l = at(lane, 8);
+            L[j * kIcwyRow + lane] = l;
+            gram[j * kIcwyMax + lane] = l;
+        }
+        __syncwarp();
+        double h = lane <= j ? at(lane, 0) : 0.0;
+        for (int i = 0; i < j; ++i) {
+            const double hi = __shfl_sync(0xffffffffu, h, i);
+            if (lane > i && lane <= j) h = __fma_rn(-L[lane * kIcwyRow + i], hi, h);
+        }
+        if (lane <= j) hcol[lane] = h;
+        if (lane == 0) *red.ticket = 0u;
+    }
+}
+
+// w -= sum_{r <= j} h_r V_r, one FMA a term in r order, and *norm = ||w||.  Two elements a thread at a time: the
+// terms of one are a chain.
+__global__ void __launch_bounds__(kRedThreads) k_icwy_update(double* __restrict__ w, const double* __restrict__ V,
+                                                             size_t N, int j, const double* __restrict__ hcol,
+                                                             RedArgs red, double* norm) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ double h[kIcwyMax];
+    __shared__ double sm[1][32];
+    if (threadIdx.x <= j) h[threadIdx.x] = hcol[threadIdx.x];
+    __syncthreads();
+    double s[1] = {0.0};
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += 2 * stride) {
+        const size_t i2 = i + stride;
+        const bool two = i2 < N;
+        double wa = w[i], wb = two ? w[i2] : 0.0;
+        const double *va = V + i, *vb = V + (two ? i2 : i);
+#pragma unroll 4
+        for (int r = 0; r <= j; ++r, va += N, vb += N) {
+            wa = __fma_rn(-h[r], *va, wa);
+            wb = __fma_rn(-h[r], *vb, wb);
+        }
+        w[i] = wa;
+        s[0] = __fma_rn(wa, wa, s[0]);
+        if (two) {
+            w[i2] = wb;
+            s[0] = __fma_rn(wb, wb, s[0]);
+        }
+    }
+    block_sum<1>(s, sm);
+    grid_reduce_finish<1>(s, red, StoreSqrtAt{norm});
+}
+
+// vnext = w / d with the norm d on the device, as k_div forms it (0 where d is not positive), so the host reads
+// the column after the kernel is launched.
+__global__ void k_div_dev(const double* __restrict__ w, const double* __restrict__ d, double* __restrict__ vnext,
+                          size_t N) {
+    pdl_wait();
+    pdl_trigger();
+    const double dv = *d, rd = dv > 0.0 ? __ddiv_rn(1.0, dv) : 0.0;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += stride)
+        vnext[i] = dv > 0.0 ? w[i] * rd : 0.0;
 }
 
 // CGS2 pieces.  V is (j+1) consecutive vectors of length ldv.
@@ -577,6 +741,20 @@ void Gmres::arnoldi_mgs(size_t j, double* w) {
     const size_t N = N_;
     const unsigned g = ctx_.red_grid(N);
     const double* V = V_.p;
+    if (j >= (size_t)kIcwyFrom && j < (size_t)kIcwyMax && N <= kIcwyMaxN) {
+        gram_.resize(kIcwyMax * kIcwyMax);
+        const size_t blocks = (N + 2 * kRedThreads - 1) / (2 * kRedThreads);
+        // two blocks an SM for the inner products: each block's partial sums are 16 more values for the last one
+        const unsigned gd = (unsigned)std::min<size_t>(blocks, 2 * (size_t)ctx_.sm_count);
+        const bool start = j == (size_t)kIcwyFrom;
+        launch_pdl(start ? k_icwy_dots<true> : k_icwy_dots<false>, dim3(gd, (unsigned)(j / 8 + 1 + start)), kRedThreads, 0,
+                   ctx_.stream, (const double*)w, V, N, (int)j, ctx_.red, gram_.p, hcol);
+        launch_pdl(k_icwy_update, (unsigned)std::min<size_t>(blocks, 8 * (size_t)ctx_.sm_count), kRedThreads, 0,
+                   ctx_.stream, w, V, N, (int)j, (const double*)hcol, ctx_.red, hcol + j + 1);
+        ctx_.count_launch(2);
+        ctx_.check_launch("arnoldi mgs");
+        return;
+    }
     launch_pdl(k_mgs<false, false, StoreAt>, g, kRedThreads, 0, ctx_.stream, w, nullptr, nullptr, V, N, ctx_.red, StoreAt{hcol});
     ctx_.count_launch();
     for (size_t i = 1; i <= j; ++i) {
@@ -967,24 +1145,20 @@ GmresResult Gmres::solve(LinearOp& A, Precond* M, const double* b, double* x, co
             ++res.matvecs;
             if (cgs2) {
                 arnoldi_cgs2(j, w_.p);
-                ctx_.fetch(sl, (int)(j + 2), col.data());
-                ctx_.fetch(ctx_.scalar(kSlotGmresH2), (int)(j + 1), col2.data());
-                for (size_t i = 0; i <= j; ++i) col[i] += col2[i];
             } else if (cgs1) {
                 arnoldi_cgs1(j, w_.p);
-                ctx_.fetch(sl, (int)(j + 2), col.data());
             } else {
                 arnoldi_mgs(j, w_.p);
-                ctx_.fetch(sl, (int)(j + 2), col.data());
+            }
+            launch_pdl(k_div_dev, eg, 256, 0, ctx_.stream, (const double*)w_.p, (const double*)(sl + j + 1),
+                       V_.p + (j + 1) * N, N);
+            ctx_.count_launch();
+            ctx_.fetch(sl, (int)(j + 2), col.data());
+            if (cgs2) {
+                ctx_.fetch(ctx_.scalar(kSlotGmresH2), (int)(j + 1), col2.data());
+                for (size_t i = 0; i <= j; ++i) col[i] += col2[i];
             }
             for (size_t i = 0; i <= j + 1; ++i) H[i][j] = col[i];
-            double* vnext = V_.p + (j + 1) * N;
-            if (H[j + 1][j] > 0.0) {
-                launch_pdl(k_div, eg, 256, 0, ctx_.stream, w_.p, H[j + 1][j], 1.0 / H[j + 1][j], vnext, N);
-                ctx_.count_launch();
-            } else {
-                dev_fill(ctx_, vnext, 0.0, N);
-            }
             for (size_t i = 0; i <= j + 1; ++i) Hraw[i][j] = H[i][j];
             for (size_t i = 0; i < j; ++i) {
                 const double t = cs[i] * H[i][j] + sn[i] * H[i + 1][j];

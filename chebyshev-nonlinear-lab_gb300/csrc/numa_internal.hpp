@@ -616,6 +616,7 @@ private:
     Context& ctx_;
     size_t N_;
     DeviceArray<double> V_, Z_, w_, r_, comb_, z_, rrec_;
+    DeviceArray<double> gram_;  // strictly lower part of V^T V of the current cycle (MGS in compact WY form)
     DeviceArray<float> Z32_;  // FGMRES preconditioned vectors in FP32 (FP32 preconditioner and product)
     DeviceArray<float> V32_;  // FGMRES basis in FP32 (FP32 hand-off, loose linear tolerance)
     DeviceArray<float> W32_;  // its A z_j in FP32
