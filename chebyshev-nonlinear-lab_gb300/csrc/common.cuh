@@ -495,7 +495,9 @@ struct Context {
     cudaStream_t stream = nullptr;
     RedArgs red{};
     double* d_scalars = nullptr;  // kNumScalars device scalars
-    double* h_scalars = nullptr;  // pinned host mirror
+    double* h_scalars = nullptr;  // pinned host mirror, written by the device; the last word is its sequence number
+    double* h_scalars_dev = nullptr;  // its device address
+    unsigned long long fetch_seq = 0;
     cudaEvent_t done = nullptr;
     uint64_t launches = 0;
     bool timing = false;
@@ -507,7 +509,7 @@ struct Context {
     Context& operator=(const Context&) = delete;
 
     void sync();
-    // Copies count device doubles to host memory and waits for them.
+    // Copies count device doubles to host memory and waits for them (and for all earlier work on the stream).
     void fetch(const double* dsrc, int count, double* host);
     double fetch1(const double* dsrc) {
         double v;
