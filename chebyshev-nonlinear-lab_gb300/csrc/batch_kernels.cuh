@@ -20,7 +20,7 @@
 // linear solve has ended, costs its blocks an early exit.
 #pragma once
 
-#include "mg_kernels.cuh"
+#include "mg_chain.cuh"
 
 namespace numa::gpu {
 namespace {
@@ -122,16 +122,22 @@ __global__ void __launch_bounds__(BX* BY) k_bprolong(MgPool C, MgPool F, const i
                                   blockIdx.z - q * (nc + 1));
 }
 
-// the levels n <= 15 of every pool grid: one CTA per grid.  With tp.c set (Jacobian-aware tail), level m's
-// coefficients of grid q are at tp.c[m] + q n_m^3.
-__global__ void __launch_bounds__(1024) k_btail(MgPool P, const int* __restrict__ act, TailParams tp) {
+// the levels n <= 15 of every pool grid: one CTA per grid.  SHIFT (Jacobian-aware tail): level m's coefficients of
+// grid q are at io.c[m] + q n_m^3.
+template <bool SHIFT>
+__global__ void __launch_bounds__(kChainThreads, 1) k_btail(MgPool P, const int* __restrict__ act,
+                                                            const __grid_constant__ ChainIo io) {
+    using K = Chain32<false, SHIFT>;
+    chain_clear_below31<K>();
     pdl_wait();
     pdl_trigger();
     const int q = blockIdx.x;
     if (!pool_active(P, act, q)) return;
-    if (tp.c[0])
-        for (int m = 0; m < tp.levels; ++m) tp.c[m] += (size_t)q * tp.n[m] * tp.n[m] * tp.n[m];
-    mg_tail_body<float, true>(P.b + q * P.sb, P.bs + q * P.sb, P.x + q * P.sx, tp);
+    chain_load_top<typename K::L15>(io, P.b + q * P.sb, 15, 0);
+    chain_coefs<K, SHIFT>(io, q);
+    __syncthreads();
+    chain_solo15<K, SHIFT>(io, SHIFT ? io.c[3] + q : nullptr);
+    chain_store_top<typename K::L15>(io, P.x + q * P.sx, 15, 0);
 }
 
 // The Jacobian coefficient of grids g0 .. of a coarse level: the full-weighting restriction of the

@@ -568,15 +568,9 @@ void BatchSolver::Impl::alloc_state() {
         ctail[1].resize((size_t)Kt * 27);
         ctail[2].resize((size_t)Kt);
     }
-    // the tail: levels 15, 7, 3, 1 of every instance in one CTA each (and, Jacobian-aware, c h^2 of each)
-    size_t elems = 0;
-    for (int s = 15; s >= 1; s = (s - 1) / 2) {
-        elems += (jac_tail ? 4 : 3) * (size_t)s * s * s;
-        if (s == 1) break;
-    }
-    elems += 15 * 15 * 15;
-    tail_smem = elems * sizeof(float);
-    const int lim = set_dynamic_smem_limit(ctx, k_btail);
+    // the tail: levels 15, 7, 3, 1 of every instance in one CTA each
+    tail_smem = (jac_tail ? Chain32<false, true>::TOTAL : Chain32<false, false>::TOTAL) * sizeof(float);
+    const int lim = jac_tail ? set_dynamic_smem_limit(ctx, k_btail<true>) : set_dynamic_smem_limit(ctx, k_btail<false>);
     if (tail_smem > (size_t)lim) throw Status(NUMA_GPU_ERR_NOT_SUPPORTED, "batched multigrid tail exceeds shared memory");
     ctx.sync();
 }
@@ -760,22 +754,11 @@ void BatchSolver::Impl::vcycle(int j) {
     // the tail of every grid
     {
         Pool& P = *pools[np - 1];
-        TailParams tp{};
-        int l = 0;
-        for (int sz = 15; l < kMaxTail; sz = (sz - 1) / 2) {
-            const double h2 = ((double)sz + 1.0) * ((double)sz + 1.0);
-            tp.n[l] = sz;
-            tp.h2inv[l] = h2;
-            tp.inv[l] = 1.0 / h2;
-            tp.six_h2inv[l] = 6.0 * h2;
-            ++l;
-            if (sz == 1) break;
-        }
-        tp.levels = l;
+        ChainIo tp{};
+        tp.in_kind = kChainSplit;
         tp.pre = pre;
         tp.post = post;
         tp.half = make_split(15).half;
-        for (int m2 = 0; m2 < kMaxTail; ++m2) tp.c[m2] = nullptr;
         const MgPool V = P.view();
         for (int a = 0; a < P.K; a += 65535) {
             MgPool W = V;
@@ -783,14 +766,15 @@ void BatchSolver::Impl::vcycle(int j) {
             W.b += (long long)a * V.sb;
             W.bs += (long long)a * V.sb;
             W.inst += a;
-            TailParams ta = tp;
+            ChainIo ta = tp;
             if (jac_tail) {  // levels 15, 7, 3, 1 of grid a onwards
                 ta.c[0] = cpool[np - 1].p + (size_t)a * 3375;
                 ta.c[1] = ctail[0].p + (size_t)a * 343;
                 ta.c[2] = ctail[1].p + (size_t)a * 27;
                 ta.c[3] = ctail[2].p + (size_t)a;
             }
-            launch_pdl(k_btail, std::min(65535, P.K - a), 1024, tail_smem, s, W, act, ta);
+            launch_pdl(jac_tail ? k_btail<true> : k_btail<false>, std::min(65535, P.K - a), kChainThreads, tail_smem, s, W,
+                       act, ta);
             ctx.count_launch();
         }
     }

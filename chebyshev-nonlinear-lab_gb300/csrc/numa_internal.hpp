@@ -399,8 +399,14 @@ private:
     size_t tail_l_ = SIZE_MAX;
     size_t tail_smem_ = 0;
     void launch_tail32();
-    // FP64 cycle: the levels from cl_l_ down run in one kernel (mg_coarse.cuh); SIZE_MAX = none.
+    // The levels from cl_l_ down run in one kernel: mg_chain.cuh where every grid is 2^k - 1 (chain_), else, in FP64,
+    // mg_coarse.cuh; SIZE_MAX = none.
     size_t cl_l_ = SIZE_MAX;
+    bool chain_ = false;
+    void plan_chain();
+    const void* chain_kernel(bool shift) const;
+    size_t chain_smem(bool shift) const;
+    void launch_chain();
     size_t coarse_params(size_t l, CoarseParams& cp) const;
     void plan_coarse();
     void launch_coarse(const double* b, double* x);

@@ -24,6 +24,7 @@
 #include <limits>
 #include <type_traits>
 
+#include "mg_chain.cuh"
 #include "mg_coarse.cuh"
 
 namespace numa::gpu {
@@ -95,8 +96,9 @@ PoissonMG::PoissonMG(Context& ctx, size_t n, int pre, int post, int precision, i
         m = (m - 1) / 2;
         h2 /= 4.0;
     }
+    plan_chain();
     if (precision == NUMA_GPU_FP64) {
-        plan_coarse();
+        if (cl_l_ == SIZE_MAX) plan_coarse();
         for (size_t l = 0; l < levels_.size() && l <= cl_l_; ++l) {  // below, the levels live in shared memory
             Level& L = *levels_[l];
             const size_t Nl = (size_t)L.n * L.n * L.n;
@@ -175,6 +177,80 @@ cudaLaunchConfig_t coarse_config(cudaLaunchAttribute (&attr)[2], int cluster, si
 
 }  // namespace
 
+// The compile-time chain (mg_chain.cuh) takes over at 31^3 (FP32) or 15^3 (FP64) when every grid from there is 2^k - 1
+// down to one point and both smoothings sweep: V-cycles at 31^3 / 63^3 / 127^3 in FP32 take 26 / 44 / 86 us instead of
+// 45 / 63 / 100 with launched levels and k_mg_tail, at 15^3 / 31^3 / 63^3 in FP64 29 / 57 / 105 instead of 37 / 64 / 111
+// with the coarse kernel of runtime sizes.
+void PoissonMG::plan_chain() {
+    const int top = precision_ == NUMA_GPU_FP64 ? 15 : 31;
+    size_t l = 0;
+    while (l < levels_.size() && levels_[l]->n != top) ++l;
+    if (l == levels_.size() || pre_ == 0 || post_ == 0) return;
+    for (size_t m = l; m < levels_.size(); ++m) {  // (31 and 15 halve to odd grids down to one point)
+        const double n1 = levels_[m]->n + 1.0;
+        if (levels_[m]->h2inv != n1 * n1) return;  // the kernel's constants
+    }
+    if (levels_.back()->n != 1) return;  // a capped hierarchy
+    const void* kern = chain_kernel(true);
+    if (chain_smem(true) > (size_t)smem_optin_limit(ctx_)) return;
+    for (const bool shift : {false, true}) {
+        kern = chain_kernel(shift);
+        NUMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chain_smem(shift)));
+    }
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = coarse_config(attr, kChainCluster, chain_smem(true), ctx_.stream);
+    int clusters = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
+    if (e != cudaSuccess || clusters < 1) {
+        cudaGetLastError();
+        return;
+    }
+    cl_l_ = l;
+    chain_ = true;
+}
+
+const void* PoissonMG::chain_kernel(bool shift) const {
+    if (precision_ == NUMA_GPU_FP64) return reinterpret_cast<const void*>(k_chain64);
+    return shift ? reinterpret_cast<const void*>(k_chain32<true>) : reinterpret_cast<const void*>(k_chain32<false>);
+}
+
+size_t PoissonMG::chain_smem(bool shift) const {
+    if (precision_ == NUMA_GPU_FP64) return Chain64::TOTAL * sizeof(double);
+    return (shift ? Chain32<true, true>::TOTAL : Chain32<true, false>::TOTAL) * sizeof(float);
+}
+
+// The cycle from level cl_l_ down through the chain kernel.
+void PoissonMG::launch_chain() {
+    Level& L = *levels_[cl_l_];
+    ChainIo io{};
+    io.pre = pre_;
+    io.post = post_;
+    io.half = make_split(L.n).half;
+    const bool fp64 = precision_ == NUMA_GPU_FP64, finest = cl_l_ == 0, shift = !fp64 && coarse_jac_;
+    if (fp64) {
+        io.in_kind = kChainSame;
+        io.b = finest ? b0_ : L.b64.p;
+        io.x_nat = finest ? x0_ : L.x64.p;
+    } else if (finest) {
+        io.in_kind = in32_ ? kChainSame : kChainF64;
+        io.b = in32_ ? static_cast<const void*>(in32_) : b0_;
+        io.x_nat = z32_out_;
+        io.z64 = z0_;
+    } else {
+        io.in_kind = kChainSplit;
+        io.b = L.b32.p;
+        io.x_split = L.cur32 = L.xs;
+    }
+    if (shift)
+        for (int m = 0; m < 4; ++m) io.c[m] = cl_.p + cl_off_[cl_l_ + 1 + m];
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = coarse_config(attr, kChainCluster, chain_smem(shift), ctx_.stream);
+    void* args[] = {&io};
+    NUMA_CUDA(cudaLaunchKernelExC(&cfg, chain_kernel(shift), args));
+    ctx_.count_launch();
+    ctx_.check_launch("mg chain");
+}
+
 // The coarse kernel's parameters for the FP64 cycle from level l down; returns its shared memory in bytes.
 size_t PoissonMG::coarse_params(size_t l, CoarseParams& cp) const {
     int n[kCoarseMax];
@@ -229,7 +305,8 @@ PoissonMG::~PoissonMG() {
 
 void PoissonMG::coarse_cycle() {
     if (cl_l_ == 1) {  // one kernel: no graph
-        launch_coarse(levels_[1]->b64.p, levels_[1]->x64.p);
+        if (chain_) launch_chain();
+        else launch_coarse(levels_[1]->b64.p, levels_[1]->x64.p);
         return;
     }
     if (coarse_exec_ && graph_jac_ != coarse_jac_) {  // captured in the other tail mode
@@ -267,7 +344,8 @@ template <class T>
 void PoissonMG::cycle(size_t l) {
     Level& L = *levels_[l];
     if (l == cl_l_) {
-        launch_coarse(L.b64.p, L.x64.p);
+        if (chain_) launch_chain();
+        else launch_coarse(L.b64.p, L.x64.p);
         return;
     }
     const int n = L.n;
@@ -354,12 +432,16 @@ void PoissonMG::cycle(size_t l) {
 // True when level l's first smoothing pass is fused into the producer of its right-hand side.
 bool PoissonMG::first_fused32(size_t l) const {
     const Level& L = *levels_[l];
-    if (!(L.n & 1) || l == tail_l_) return false;
+    if (!(L.n & 1) || l == tail_l_ || l == cl_l_) return false;
     if (l + 1 == levels_.size()) return L.n > 1;  // coarsest: 30 sweeps, the first from x = 0
     return pre_ > 0;
 }
 
 void PoissonMG::cycle32(size_t l) {
+    if (l == cl_l_) {
+        launch_chain();
+        return;
+    }
     if (l == tail_l_) {
         launch_tail32();
         return;
@@ -495,7 +577,10 @@ void PoissonMG::apply(const double* r, double* z) {
     const size_t N = N0_;
     if (precision_ == NUMA_GPU_FP64) {
         if (cl_l_ == 0) {  // (r and z may be the same vector)
-            launch_coarse(r, z);
+            b0_ = r;
+            x0_ = z;
+            if (chain_) launch_chain();
+            else launch_coarse(r, z);
             return;
         }
         const double* b = r;
@@ -511,6 +596,10 @@ void PoissonMG::apply(const double* r, double* z) {
         bs0_ = L0.bs64.p;
         z0_ = nullptr;
         cycle<double>(0);
+    } else if (cl_l_ == 0) {
+        b0_ = r;
+        z0_ = z;
+        launch_chain();
     } else {
         auto scale_in = [&](auto rin) {
             using RT = std::remove_cv_t<std::remove_pointer_t<decltype(rin)>>;
