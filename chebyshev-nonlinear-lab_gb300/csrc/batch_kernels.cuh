@@ -122,22 +122,33 @@ __global__ void __launch_bounds__(BX* BY) k_bprolong(MgPool C, MgPool F, const i
                                   blockIdx.z - q * (nc + 1));
 }
 
-// the levels n <= 15 of every pool grid: one CTA per grid.  SHIFT (Jacobian-aware tail): level m's coefficients of
-// grid q are at io.c[m] + q n_m^3.
+// 31^3 and below of every grid of the 31^3 pool: a cluster of 8 CTAs a grid (mg_chain.cuh).  The first top0 grids
+// take b from the pool and leave x there; the others are their instances' finest level: b is their basis vector (u +
+// (q - top0) N) and x their preconditioned vector (z + ...).  SHIFT (Jacobian-aware levels): level m's coefficients
+// of grid q are at io.c[m] + q n_m^3.
 template <bool SHIFT>
-__global__ void __launch_bounds__(kChainThreads, 1) k_btail(MgPool P, const int* __restrict__ act,
-                                                            const __grid_constant__ ChainIo io) {
-    using K = Chain32<false, SHIFT>;
-    chain_clear_below31<K>();
+__global__ void __launch_bounds__(kChainThreads, 1) k_bchain(MgPool P, const int* __restrict__ act, int top0,
+                                                             const float* __restrict__ u, float* __restrict__ z,
+                                                             const __grid_constant__ ChainIo io) {
+    using K = Chain32<SHIFT>;
+    using L31 = typename K::L31;
+    constexpr long long N = 31 * 31 * 31;
+    const int rank = (int)cooperative_groups::this_cluster().block_rank(), my = min(4, 31 - 4 * rank);
+    chain_clear<L31>();
+    if (rank == 0) chain_clear_below31<K>();
+    cooperative_groups::this_cluster().sync();
     pdl_wait();
     pdl_trigger();
-    const int q = blockIdx.x;
-    if (!pool_active(P, act, q)) return;
-    chain_load_top<typename K::L15>(io, P.b + q * P.sb, 15, 0);
-    chain_coefs<K, SHIFT>(io, q);
+    const int q = blockIdx.x / kChainCluster;
+    if (!pool_active(P, act, q)) return;  // (the whole cluster)
+    const bool finest = q >= top0;
+    chain_load_top<L31>(finest ? kChainSame : kChainSplit, io.half, finest ? u + (q - top0) * N : P.b + q * P.sb, my, rank);
+    if (rank == 0) chain_coefs<K, SHIFT>(io, q);
     __syncthreads();
-    chain_solo15<K, SHIFT>(io, SHIFT ? io.c[3] + q : nullptr);
-    chain_store_top<typename K::L15>(io, P.x + q * P.sx, 15, 0);
+    chain_cycle31<SHIFT>(io, SHIFT ? io.c[3] + q : nullptr, my, rank);
+    chain_store_top<L31>(io.half, finest ? nullptr : P.x + q * P.sx, finest ? z + (q - top0) * N : nullptr, nullptr, my,
+                         rank);
+    cooperative_groups::this_cluster().sync();
 }
 
 // The Jacobian coefficient of grids g0 .. of a coarse level: the full-weighting restriction of the
@@ -569,9 +580,9 @@ __global__ void __launch_bounds__(kEwThreads) k_bscale32(const double* __restric
         u0[i] = f64_to_f32(__dmul_rn(r[i], s));
 }
 
-// Per-instance sums of block partials, in block order: out[t * ostride + ooff + r] = sum over the
-// instance's partial slots [p0[t], p0[t] + pn[t]) of partials[slot * R + r], for r < R.  One warp per
-// instance; lane r sums result r.
+// Per-instance sums of block partials: out[t * ostride + ooff + r] = sum over the instance's partial slots
+// [p0[t], p0[t] + pn[t]) of partials[slot * R + r], for r < R <= 8.  One warp per instance; its lanes share out the
+// slots (in an order that depends on R and pn alone): one lane a result took 26 us for 130 slots.
 __global__ void k_bsegsum(const double* __restrict__ partials, int R, const int* __restrict__ p0,
                           const int* __restrict__ pn, const int* __restrict__ act, int I, double* __restrict__ out,
                           int ostride, int ooff) {
@@ -579,11 +590,15 @@ __global__ void k_bsegsum(const double* __restrict__ partials, int R, const int*
     pdl_trigger();
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
-    if (t >= I || !act[t] || lane >= R) return;
+    if (t >= I || !act[t]) return;
+    // one result: 32 lanes on it; more: 4 lanes each
+    const int per = R == 1 ? 32 : 4, r = R == 1 ? 0 : lane >> 2, part = R == 1 ? lane : lane & 3;
     double s = 0.0;
     const int b0 = p0[t], nb = pn[t];
-    for (int b = 0; b < nb; ++b) s += partials[(size_t)(b0 + b) * R + lane];
-    out[(long long)t * ostride + ooff + lane] = s;
+    if (r < R)
+        for (int b = part; b < nb; b += per) s += partials[(size_t)(b0 + b) * R + r];
+    for (int o = per >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (r < R && part == 0) out[(long long)t * ostride + ooff + r] = s;
 }
 
 }  // namespace

@@ -354,7 +354,7 @@ struct BatchSolver::Impl {
         }
     };
     std::vector<std::unique_ptr<Pool>> pools;  // sizes n_max ... 15 (the last one is the tail)
-    size_t tail_smem = 0;
+    size_t chain_smem = 0;
     // Jacobian-aware tail (kp.coarse_jacobian): the coefficient c = lambda e^u of each pool grid below the
     // finest pool (natural layout, grid q at q s^3), and of the tail's levels 7, 3, 1 (grid q of the last pool)
     bool jac_tail = false;
@@ -531,7 +531,8 @@ void BatchSolver::Impl::alloc_state() {
         std::lock_guard<std::recursive_mutex> lk(alloc_capture_mutex());
         NUMA_CUDA(cudaMallocHost(reinterpret_cast<void**>(&flags_h), sizeof(int)));
     }
-    // multigrid pools: sizes n_max, (n_max - 1) / 2, ..., 15
+    // multigrid pools: sizes n_max, (n_max - 1) / 2, ..., 31 and 15 (whose levels live in the chain kernel: only its
+    // instances and coefficients are kept)
     std::vector<int> top_of_size;
     for (int s = cls.front().n; s >= 15; s = (s - 1) / 2) {
         auto P = std::make_unique<Pool>();
@@ -548,16 +549,19 @@ void BatchSolver::Impl::alloc_state() {
                 P->cls = c;
                 P->top0 = P->K - cls[c].count;
             }
-        P->x.resize((size_t)P->K * (P->N + 2 * P->pad));
-        P->b.resize((size_t)P->K * (P->N + 64));
-        P->bs.resize((size_t)P->K * (P->N + 64));
-        if (s > 15) P->r.resize((size_t)P->K * P->N);
+        if (s > 15) {
+            P->x.resize((size_t)P->K * (P->N + 2 * P->pad));
+            P->b.resize((size_t)P->K * (P->N + 64));
+            P->bs.resize((size_t)P->K * (P->N + 64));
+        }
+        if (s > 31) P->r.resize((size_t)P->K * P->N);
         P->inst.resize(P->K);
         NUMA_CUDA(cudaMemcpyAsync(P->inst.p, insts.data(), P->K * sizeof(int), cudaMemcpyHostToDevice, ctx.stream));
-        // padding and untouched halves read by the unconditional loads must be finite
-        NUMA_CUDA(cudaMemsetAsync(P->x.p, 0, P->x.n * sizeof(float), ctx.stream));
-        NUMA_CUDA(cudaMemsetAsync(P->b.p, 0, P->b.n * sizeof(float), ctx.stream));
-        NUMA_CUDA(cudaMemsetAsync(P->bs.p, 0, P->bs.n * sizeof(float), ctx.stream));
+        if (s > 15) {  // padding and untouched halves read by the unconditional loads must be finite
+            NUMA_CUDA(cudaMemsetAsync(P->x.p, 0, P->x.n * sizeof(float), ctx.stream));
+            NUMA_CUDA(cudaMemsetAsync(P->b.p, 0, P->b.n * sizeof(float), ctx.stream));
+            NUMA_CUDA(cudaMemsetAsync(P->bs.p, 0, P->bs.n * sizeof(float), ctx.stream));
+        }
         pools.push_back(std::move(P));
     }
     if (jac_tail) {
@@ -568,16 +572,19 @@ void BatchSolver::Impl::alloc_state() {
         ctail[1].resize((size_t)Kt * 27);
         ctail[2].resize((size_t)Kt);
     }
-    // the tail: levels 15, 7, 3, 1 of every instance in one CTA each
-    tail_smem = (jac_tail ? Chain32<false, true>::TOTAL : Chain32<false, false>::TOTAL) * sizeof(float);
-    const int lim = jac_tail ? set_dynamic_smem_limit(ctx, k_btail<true>) : set_dynamic_smem_limit(ctx, k_btail<false>);
-    if (tail_smem > (size_t)lim) throw Status(NUMA_GPU_ERR_NOT_SUPPORTED, "batched multigrid tail exceeds shared memory");
+    // 31^3 and below of every instance: one cluster each
+    chain_smem = (jac_tail ? Chain32<true>::TOTAL : Chain32<false>::TOTAL) * sizeof(float);
+    const int lim = jac_tail ? set_dynamic_smem_limit(ctx, k_bchain<true>) : set_dynamic_smem_limit(ctx, k_bchain<false>);
+    if (chain_smem > (size_t)lim) throw Status(NUMA_GPU_ERR_NOT_SUPPORTED, "batched multigrid exceeds shared memory");
     ctx.sync();
 }
 
 void BatchSolver::Impl::build_tables() {
     // element-wise block table
-    const long long E = std::max(1024, tune.elems_per_block);
+    // at least eight blocks an SM where the batch is small: at 32,768 elements a block 32 instances of 31^3 and 63^3
+    // made 100 blocks, and a Gram-Schmidt pass over four vectors took 79 us
+    const long long fill = std::max<long long>(2048, T / (8LL * ctx.sm_count) / 1024 * 1024);
+    const long long E = std::min<long long>(std::max(1024, tune.elems_per_block), fill);
     std::vector<int> bi, b0(I), bn(I);
     std::vector<long long> bb, be;
     for (int t = 0; t < I; ++t) {
@@ -677,25 +684,30 @@ void BatchSolver::Impl::vcycle(int j) {
         const Split g = make_split(P.s);
         const MgPool V = P.view();
         const int n = P.s;
-        const int zch = n >= 64 ? (n + 3) / 4 : n;
+        // four planes a thread above 63^3, and at 63^3 from eight resident blocks an SM on (one plane a thread there
+        // gives 504 blocks a grid: several waves of very short blocks)
+        const bool four = n >= 64 || (n == 63 && (long long)count * 128 >= 8LL * ctx.sm_count);
+        const int zch = four ? (n + 3) / 4 : n;
         const dim3 grid0(((n + 1) / 2 + BX - 1) / BX, (n + BY - 1) / BY, 1);
         over_pool(g0, count, zch, [&](int a, int cnt) {
             const dim3 grid(grid0.x, grid0.y, cnt * zch);
             float* zq = z32 ? z32 + (long long)(a - g0) * zs : nullptr;
             if (mode == kPassLastZ) {
-                if (n >= 64) launch_pdl(k_bpass<kPassLastZ, 4, 0>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
+                if (four && n == 63) launch_pdl(k_bpass<kPassLastZ, 4, 63>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
+                else if (four) launch_pdl(k_bpass<kPassLastZ, 4, 0>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
                 else launch_pdl(k_bpass<kPassLastZ, 1, 0>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
             } else {
                 if (n == 127) launch_pdl(k_bpass<kPassFull, 4, 127>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
                 else if (n == 255) launch_pdl(k_bpass<kPassFull, 4, 255>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
-                else if (n >= 64) launch_pdl(k_bpass<kPassFull, 4, 0>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
+                else if (four && n == 63) launch_pdl(k_bpass<kPassFull, 4, 63>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
+                else if (four) launch_pdl(k_bpass<kPassFull, 4, 0>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
                 else launch_pdl(k_bpass<kPassFull, 1, 0>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
             }
             ctx.count_launch();
         });
     };
     // down: right-hand sides, pre-smoothing, residual, restriction
-    for (int p = 0; p + 1 < np; ++p) {
+    for (int p = 0; p + 2 < np; ++p) {
         Pool& P = *pools[p];
         const int n = P.s;
         const Split g = make_split(n);
@@ -733,7 +745,7 @@ void BatchSolver::Impl::vcycle(int j) {
         Pool& C = *pools[p + 1];
         const int nc = C.s;
         const Split gc = make_split(nc);
-        const bool fused = (p + 2 < np);  // the tail level's first pass is its own
+        const bool fused = (p + 3 < np);  // the first pass at 31^3 is the chain's own
         const MgPool CV = C.view();
         const int zc = (nc + 1) / 2;  // two coarse planes a thread
         over_pool(0, P.K, zc, [&](int a, int cnt) {
@@ -751,35 +763,37 @@ void BatchSolver::Impl::vcycle(int j) {
             ctx.count_launch();
         });
     }
-    // the tail of every grid
+    // 31^3 and below of every grid
     {
-        Pool& P = *pools[np - 1];
-        ChainIo tp{};
-        tp.in_kind = kChainSplit;
-        tp.pre = pre;
-        tp.post = post;
-        tp.half = make_split(15).half;
-        const MgPool V = P.view();
-        for (int a = 0; a < P.K; a += 65535) {
-            MgPool W = V;
-            W.x += (long long)a * V.sx;
-            W.b += (long long)a * V.sb;
-            W.bs += (long long)a * V.sb;
-            W.inst += a;
-            ChainIo ta = tp;
-            if (jac_tail) {  // levels 15, 7, 3, 1 of grid a onwards
-                ta.c[0] = cpool[np - 1].p + (size_t)a * 3375;
-                ta.c[1] = ctail[0].p + (size_t)a * 343;
-                ta.c[2] = ctail[1].p + (size_t)a * 27;
-                ta.c[3] = ctail[2].p + (size_t)a;
-            }
-            launch_pdl(jac_tail ? k_btail<true> : k_btail<false>, std::min(65535, P.K - a), kChainThreads, tail_smem, s, W,
-                       act, ta);
-            ctx.count_launch();
+        Pool& P = *pools[np - 2];
+        ChainIo io{};
+        io.pre = pre;
+        io.post = post;
+        io.half = make_split(31).half;
+        if (jac_tail) {
+            io.c[0] = cpool[np - 1].p;
+            for (int m2 = 0; m2 < 3; ++m2) io.c[m2 + 1] = ctail[m2].p;
         }
+        const long long off = P.cls >= 0 ? cls[P.cls].off0 : 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)P.K * kChainCluster);
+        cfg.blockDim = dim3(kChainThreads);
+        cfg.dynamicSmemBytes = chain_smem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kChainCluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        NUMA_CUDA(cudaLaunchKernelEx(&cfg, jac_tail ? k_bchain<true> : k_bchain<false>, P.view(), act, P.top0, u + off,
+                                     zout + off, io));
+        ctx.count_launch();
     }
     // up: prolongation and post-smoothing; the finest level of each instance writes z_j
-    for (int p = np - 2; p >= 0; --p) {
+    for (int p = np - 3; p >= 0; --p) {
         Pool& P = *pools[p];
         Pool& C = *pools[p + 1];
         const int n = P.s, nc = C.s;

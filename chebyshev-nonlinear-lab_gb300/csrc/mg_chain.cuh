@@ -374,7 +374,7 @@ __device__ __forceinline__ void chain_tail(const ChainIo& io, const float* c1) {
 
 // The top level's b from global memory, x to it: a thread's own points, all loads ahead of the stores.
 template <class L>
-__device__ __noinline__ void chain_load_top(const ChainIo& io, const void* b, int my, int rank) {
+__device__ __noinline__ void chain_load_top(int in_kind, int half, const void* b, int my, int rank) {
     using T = typename L::T;
     const ChainCol<L> col;
     if (col.g >= L::G) return;
@@ -386,8 +386,8 @@ __device__ __noinline__ void chain_load_top(const ChainIo& io, const void* b, in
             const int li = col.g + u * L::G, g = ((rank * L::PL + li) * L::N + col.j) * L::N + 2 * col.kk + e;
             v[u][e] = zero<T>();
             if (li >= my || (e && col.kk == L::NP - 1)) continue;
-            if (sizeof(T) == 4 && io.in_kind == kChainF64) v[u][e] = (T)f64_to_f32(static_cast<const double*>(b)[g]);
-            else v[u][e] = static_cast<const T*>(b)[io.in_kind == kChainSplit ? split_at(g, io.half) : g];
+            if (sizeof(T) == 4 && in_kind == kChainF64) v[u][e] = (T)f64_to_f32(static_cast<const double*>(b)[g]);
+            else v[u][e] = static_cast<const T*>(b)[in_kind == kChainSplit ? split_at(g, half) : g];
         }
     T* B = chain_base<T>() + L::OB;
 #pragma unroll
@@ -398,7 +398,7 @@ __device__ __noinline__ void chain_load_top(const ChainIo& io, const void* b, in
     }
 }
 template <class L>
-__device__ __noinline__ void chain_store_top(const ChainIo& io, float* x_split, int my, int rank) {
+__device__ __noinline__ void chain_store_top(int half, float* x_split, void* x_nat, double* z64, int my, int rank) {
     using T = typename L::T;
     const ChainCol<L> col;
     if (col.g >= L::G) return;
@@ -408,10 +408,10 @@ __device__ __noinline__ void chain_store_top(const ChainIo& io, float* x_split, 
         const int li = col.g + u * L::G, g0 = ((rank * L::PL + li) * L::N + col.j) * L::N + 2 * col.kk;
         const auto put = [&](int g, T v) {
             if constexpr (sizeof(T) == 4) {
-                if (x_split) x_split[split_at(g, io.half)] = v;
-                if (io.z64) io.z64[g] = f32_to_f64(v);
+                if (x_split) x_split[split_at(g, half)] = v;
+                if (z64) z64[g] = f32_to_f64(v);
             }
-            if (io.x_nat) static_cast<T*>(io.x_nat)[g] = v;
+            if (x_nat) static_cast<T*>(x_nat)[g] = v;
         };
         const int m0 = col.template member<0>(u);
         if (col.template valid<0>(u, my)) put(g0 + m0, X[L::H + col.template at<0>(u)]);
@@ -419,16 +419,16 @@ __device__ __noinline__ void chain_store_top(const ChainIo& io, float* x_split, 
     }
 }
 
-// The level tables: FP32 with 31^3 on top (TOP31) or 15^3 (a batch's pools), FP64 with 15^3 on top.
-template <bool TOP31, bool SHIFT>
+// The level tables: FP32 with 31^3 on top, FP64 with 15^3.
+template <bool SHIFT>
 struct Chain32 {
     using T = float;
     using L31 = ChainLv<float, 31, 4, true, kBarCluster, false, 0>;
-    using L15 = ChainLv<float, 15, 15, false, kBarCta, SHIFT, TOP31 ? L31::END : 0>;
+    using L15 = ChainLv<float, 15, 15, false, kBarCta, SHIFT, L31::END>;
     using L7 = ChainLv<float, 7, 7, false, kBarGroup, SHIFT, L15::END>;
     using L3 = ChainLv<float, 3, 3, false, kBarWarp, SHIFT, L7::END>;
     using L1 = ChainLv<float, 1, 1, false, kBarWarp, false, L3::END>;
-    static constexpr int OR = L1::END, TOTAL = OR + 2 * (TOP31 ? L31::H + L31::PAD : L15::H + L15::PAD);
+    static constexpr int OR = L1::END, TOTAL = OR + 2 * (L31::H + L31::PAD);
 };
 struct Chain64 {
     using T = double;
@@ -455,7 +455,7 @@ __device__ __forceinline__ void chain_clear_below31() {
     chain_clear<typename K::L1>();
 }
 
-// 15^3 and below in one CTA (FP32): q = the grid of a batch.
+// 15^3 and below in one CTA (FP32).
 template <class K, bool SHIFT>
 __device__ __forceinline__ void chain_solo15(const ChainIo& io, const float* c1) {
     using L15 = typename K::L15;
@@ -468,6 +468,7 @@ __device__ __forceinline__ void chain_solo15(const ChainIo& io, const float* c1)
     chain_sweeps<L15>(15, 0, 2 * io.post, 1, false);
 }
 
+// (q: the grid of a batch)
 template <class K, bool SHIFT>
 __device__ __forceinline__ void chain_coefs(const ChainIo& io, size_t q) {
     if constexpr (SHIFT) {
@@ -477,10 +478,23 @@ __device__ __forceinline__ void chain_coefs(const ChainIo& io, size_t q) {
     }
 }
 
+// The cycle from 31^3 (b loaded) on a cluster of 8, in FP32.
+template <bool SHIFT>
+__device__ __forceinline__ void chain_cycle31(const ChainIo& io, const float* c1, int my, int rank) {
+    using K = Chain32<SHIFT>;
+    using L31 = typename K::L31;
+    chain_sweeps<L31>(my, rank, 2 * io.pre, 0, true);
+    chain_restrict<L31, typename K::L15, K::OR>(my, rank);
+    if (rank == 0) chain_solo15<K, SHIFT>(io, c1);
+    cooperative_groups::this_cluster().sync();
+    chain_prolong<L31, typename K::L15, K::OR>(my, rank);
+    chain_sweeps<L31>(my, rank, 2 * io.post, 1, false);
+}
+
 // 31, 15, 7, 3, 1 in FP32 on a cluster of 8
 template <bool SHIFT>
 __global__ void __launch_bounds__(kChainThreads, 1) k_chain32(const __grid_constant__ ChainIo io) {
-    using K = Chain32<true, SHIFT>;
+    using K = Chain32<SHIFT>;
     using L31 = typename K::L31;
     const int rank = (int)cooperative_groups::this_cluster().block_rank(), my = min(4, 31 - 4 * rank);
     chain_clear<L31>();
@@ -488,16 +502,11 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain32(const __grid_const
     cooperative_groups::this_cluster().sync();  // a neighbour's first halo store comes after the clearing
     pdl_wait();
     pdl_trigger();
-    chain_load_top<L31>(io, io.b, my, rank);
+    chain_load_top<L31>(io.in_kind, io.half, io.b, my, rank);
     if (rank == 0) chain_coefs<K, SHIFT>(io, 0);
     __syncthreads();
-    chain_sweeps<L31>(my, rank, 2 * io.pre, 0, true);
-    chain_restrict<L31, typename K::L15, K::OR>(my, rank);
-    if (rank == 0) chain_solo15<K, SHIFT>(io, io.c[3]);
-    cooperative_groups::this_cluster().sync();
-    chain_prolong<L31, typename K::L15, K::OR>(my, rank);
-    chain_sweeps<L31>(my, rank, 2 * io.post, 1, false);
-    chain_store_top<L31>(io, io.x_split, my, rank);
+    chain_cycle31<SHIFT>(io, SHIFT ? io.c[3] : nullptr, my, rank);
+    chain_store_top<L31>(io.half, io.x_split, io.x_nat, io.z64, my, rank);
     cooperative_groups::this_cluster().sync();  // no CTA leaves while another may write its halo
 }
 
@@ -510,7 +519,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain64(const __grid_const
     cooperative_groups::this_cluster().sync();
     pdl_wait();
     pdl_trigger();
-    chain_load_top<L15>(io, io.b, my, rank);
+    chain_load_top<L15>(io.in_kind, io.half, io.b, my, rank);
     __syncthreads();
     chain_sweeps<L15>(my, rank, 2 * io.pre, 0, true);
     chain_restrict<L15, K::L7, K::OR>(my, rank);
@@ -518,7 +527,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain64(const __grid_const
     cooperative_groups::this_cluster().sync();
     chain_prolong<L15, K::L7, K::OR>(my, rank);
     chain_sweeps<L15>(my, rank, 2 * io.post, 1, false);
-    chain_store_top<L15>(io, nullptr, my, rank);
+    chain_store_top<L15>(io.half, nullptr, io.x_nat, nullptr, my, rank);
     cooperative_groups::this_cluster().sync();
 }
 

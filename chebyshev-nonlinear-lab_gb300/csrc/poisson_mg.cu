@@ -216,7 +216,7 @@ const void* PoissonMG::chain_kernel(bool shift) const {
 
 size_t PoissonMG::chain_smem(bool shift) const {
     if (precision_ == NUMA_GPU_FP64) return Chain64::TOTAL * sizeof(double);
-    return (shift ? Chain32<true, true>::TOTAL : Chain32<true, false>::TOTAL) * sizeof(float);
+    return (shift ? Chain32<true>::TOTAL : Chain32<false>::TOTAL) * sizeof(float);
 }
 
 // The cycle from level cl_l_ down through the chain kernel.
