@@ -26,10 +26,13 @@ struct March {
 
 // Grid of (k tiles, j tiles, i chunks).  Chunks of 8 planes keep ~2M threads at n = 255; a fused
 // reduction takes 16 from n = 128 (its block sum, in FP64, is then shared by twice the points), and
-// more when it would exceed kMaxRedBlocks partials.
+// more when it would exceed kMaxRedBlocks partials.  Smaller grids halve the chunk until there are four
+// blocks an SM (152 SMs): a march of 4 planes at 31^3 left four SMs in five idle and was bound by the latency of
+// its FP64 operations (the product from x 5.8 us, with one plane a thread 2.8; with c given 4.5 and 2.5).
 March march_shape(int n, bool reducing) {
     const int kb = (n + BX - 1) / BX, jb = (n + BY - 1) / BY;
-    int ichunk = n >= 64 ? (reducing && n >= 128 ? 16 : 8) : (n >= 16 ? 4 : 1);
+    int ichunk = reducing && n >= 128 ? 16 : 8;
+    while (ichunk > 1 && (long)kb * jb * ((n + ichunk - 1) / ichunk) < 4 * 152) ichunk /= 2;
     if (reducing) {
         const long cols = (long)kb * jb;
         const long max_chunks = kMaxRedBlocks / cols;
@@ -404,14 +407,18 @@ __global__ void k_coef32(const double* __restrict__ c, float* __restrict__ c32, 
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += stride) c32[i] = f64_to_f32(c[i]);
 }
 
-// out = -c v v  (bratu3d.hpp:52: -lambda * exp(u) * v * v, evaluated left to right)
-__global__ void k_d2(const double* __restrict__ c, const double* __restrict__ v, double* __restrict__ out, size_t N) {
+// out = -c v v  (bratu3d.hpp:52: -lambda * exp(u) * v * v, evaluated left to right), with c given, or formed here from
+// x (FROM_X)
+template <bool FROM_X>
+__global__ void k_d2(const double* __restrict__ cx, const double* __restrict__ v, double* __restrict__ out, size_t N,
+                     double lam) {
     pdl_wait();
     pdl_trigger();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < N; p += stride) {
         const double vv = v[p];
-        out[p] = ((-c[p]) * vv) * vv;
+        const double c = FROM_X ? lam * exp_tang(cx[p]) : cx[p];
+        out[p] = ((-c) * vv) * vv;
     }
 }
 
@@ -662,9 +669,15 @@ void Bratu3D::jvp_x(const double* x, const double* v, double* out) {
 }
 
 void Bratu3D::d2_c(const double* c, const double* v, double* out) {
-    launch_pdl(k_d2, ew_grid(ctx_, N_), 256, 0, ctx_.stream, c, v, out, N_);
+    launch_pdl(k_d2<false>, ew_grid(ctx_, N_), 256, 0, ctx_.stream, c, v, out, N_, lambda_);
     ctx_.count_launch();
     ctx_.check_launch("bratu3d d2");
+}
+
+void Bratu3D::d2_x(const double* x, const double* v, double* out) {
+    launch_pdl(k_d2<true>, ew_grid(ctx_, N_), 256, 0, ctx_.stream, x, v, out, N_, lambda_);
+    ctx_.count_launch();
+    ctx_.check_launch("bratu3d d2(x)");
 }
 
 void Bratu3D::jacobi_diag_c(const double* c, double* d) {

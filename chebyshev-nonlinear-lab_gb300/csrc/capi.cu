@@ -217,12 +217,11 @@ void op_derivative(NonlinearOp& f, bool second, const double* x, const double* v
     Context& c = f.ctx();
     const size_t N = f.size();
     if (mode == NUMA_GPU_DERIV_FD) {
-        DeviceArray<double> f0(N);
-        f.eval(x, f0.p, nullptr, nullptr);
+        double* f0 = f.fd_f0();
+        f.eval(x, f0, nullptr, nullptr);
         dev_norm2(c, x, N, c.scalar(kSlotTmp1));
-        if (second) f.d2_fd(x, f0.p, c.scalar(kSlotTmp1), v, out);
-        else f.jvp_fd(x, f0.p, c.scalar(kSlotTmp1), v, out);
-        c.sync();
+        if (second) f.d2_fd(x, f0, c.scalar(kSlotTmp1), v, out);
+        else f.jvp_fd(x, f0, c.scalar(kSlotTmp1), v, out);
         return;
     }
     need(mode == NUMA_GPU_DERIV_ANALYTIC || (mode == NUMA_GPU_DERIV_ANALYTIC_FP32 && !second),
@@ -243,9 +242,12 @@ void op_derivative(NonlinearOp& f, bool second, const double* x, const double* v
         f.jvp_at(x, v, out);
         return;
     }
-    DeviceArray<double> cache(f.cache_size());
-    DeviceArray<double> tmp(f.cache_size() ? N : 0);
-    if (f.cache_size()) f.eval(x, tmp.p, cache.p, nullptr);
+    if (!f.cache_size()) {
+        f.d2(x, nullptr, v, out);
+        return;
+    }
+    DeviceArray<double> cache(f.cache_size()), tmp(N);
+    f.eval(x, tmp.p, cache.p, nullptr);
     f.d2(x, cache.p, v, out);
     c.sync();
 }
@@ -539,11 +541,10 @@ int numa_gpu_bratu3d_jvp(numa_gpu_bratu3d* op, const numa_gpu_vec* x, const numa
         Bratu3D& f = *op->impl;
         Context& c = *op->ctx->impl;
         if (mode == NUMA_GPU_DERIV_FD) {
-            DeviceArray<double> f0(f.size());
-            f.eval(x->d, f0.p);
+            double* f0 = f.fd_f0();
+            f.eval(x->d, f0);
             dev_norm2(c, x->d, f.size(), c.scalar(kSlotTmp1));
-            f.jvp_fd(x->d, f0.p, c.scalar(kSlotTmp1), v->d, out->d);
-            c.sync();
+            f.jvp_fd(x->d, f0, c.scalar(kSlotTmp1), v->d, out->d);
         } else if (mode == NUMA_GPU_DERIV_ANALYTIC_FP32) {
             DeviceArray<double> c64(f.size());
             DeviceArray<float> c32(f.size());
@@ -576,17 +577,15 @@ int numa_gpu_bratu3d_d2(numa_gpu_bratu3d* op, const numa_gpu_vec* x, const numa_
         need(out->d != x->d && out->d != v->d, NUMA_GPU_ERR_INVALID_ARGUMENT, "d2 output must not alias an input");
         Bratu3D& f = *op->impl;
         Context& c = *op->ctx->impl;
-        DeviceArray<double> tmp(f.size());
         if (mode == NUMA_GPU_DERIV_FD) {
-            f.eval(x->d, tmp.p);
+            double* f0 = f.fd_f0();
+            f.eval(x->d, f0);
             dev_norm2(c, x->d, f.size(), c.scalar(kSlotTmp1));
-            f.d2_fd(x->d, tmp.p, c.scalar(kSlotTmp1), v->d, out->d);
+            f.d2_fd(x->d, f0, c.scalar(kSlotTmp1), v->d, out->d);
         } else {
             need(mode == NUMA_GPU_DERIV_ANALYTIC, NUMA_GPU_ERR_INVALID_ARGUMENT, "unknown derivative mode");
-            f.coef(x->d, tmp.p);
-            f.d2_c(tmp.p, v->d, out->d);
+            f.d2_x(x->d, v->d, out->d);
         }
-        c.sync();
     });
 }
 

@@ -91,7 +91,7 @@ void Context::fetch(const double* dsrc, int count, double* host) {
     count_launch();
     const auto arrived = [&] { return __atomic_load_n(word, __ATOMIC_ACQUIRE) == seq; };
     for (unsigned spins = 0; !arrived(); ++spins) {
-        if (spins < 4096 || (spins & 255)) continue;
+        if (spins < 32768 || (spins & 255)) continue;
         // a long wait: let other threads run, and look whether the stream has failed or ended
         std::this_thread::yield();
         const cudaError_t e = cudaStreamQuery(stream);

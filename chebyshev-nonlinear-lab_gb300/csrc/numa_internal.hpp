@@ -122,6 +122,11 @@ public:
     // Finite-difference forms of operators/operator.hpp:101-134 over eval.  f0 = F(x) must be
     // supplied (the same vector the reference recomputes inside the call); xnorm = ||x|| as a
     // device scalar.
+    // Scratch for F(x) of the forms above, kept with the operator (callers without an F(x) of their own).
+    double* fd_f0() {
+        fd0_.resize(size());
+        return fd0_.p;
+    }
     void jvp_fd(const double* x, const double* f0, const double* xnorm_dev, const double* v, double* out);
     void d2_fd(const double* x, const double* f0, const double* xnorm_dev, const double* v, double* out);
 
@@ -133,7 +138,7 @@ protected:
     Context& ctx_;
 
 private:
-    DeviceArray<double> fd1_, fd2_, fd3_;  // finite-difference scratch
+    DeviceArray<double> fd0_, fd1_, fd2_, fd3_;  // finite-difference scratch
     std::unique_ptr<SolverWorkspace> ws_;
 };
 
@@ -194,6 +199,8 @@ public:
     void coef32(const double* c, float* c32);
     // out = F'(x) v computing e^x in the kernel.
     void jvp_x(const double* x, const double* v, double* out);
+    // out = F''(x)[v,v] = -lambda e^x v^2 computing e^x in the kernel.
+    void d2_x(const double* x, const double* v, double* out);
     // out = F''(x)[v,v] = -c v^2 (bratu3d.hpp:46-56).
     void d2_c(const double* c, const double* v, double* out);
     // d = 6 h^-2 - c (bratu3d.hpp:59-69).
