@@ -81,26 +81,48 @@ __device__ __forceinline__ void warp_sum_scatter(double (&v)[R]) {
     for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
 }
 
-// Block-wide sum of R values per thread; every thread of the block must call it.  Returns the
-// block totals in warp 0 lane 0 (others hold unspecified values).
+// Block-wide sum of R <= 8 values per thread; every thread of the block (at most 256) must call it.  Returns the
+// block totals in warp 0 lane 0 (others hold unspecified values).  One butterfly a warp and value, as it was, is 5
+// FP64 additions on each of eight warps; one value is instead summed from shared memory by warp 0 (12 in all), several
+// by warp_sum_scatter.
 template <int R>
 __device__ __forceinline__ void block_sum(double (&v)[R], double (*smem)[32]) {
-    const int lane = threadIdx.x & 31;
     const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
-    const int warp = tid >> 5;
-    const int nwarps = (blockDim.x * blockDim.y * blockDim.z + 31) >> 5;
+    const int nthreads = blockDim.x * blockDim.y * blockDim.z;
+    if constexpr (R == 1) {
+        __shared__ double buf[256];
+        buf[tid] = v[0];
+        __syncthreads();
+        if (tid < 32) {
+            double t[8];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        double s = warp_sum(v[r]);
-        if ((tid & 31) == 0) smem[r][warp] = s;
-    }
-    (void)lane;
-    __syncthreads();
-    if (warp == 0) {
+            for (int k = 0; k < 8; ++k) t[k] = tid + 32 * k < nthreads ? buf[tid + 32 * k] : 0.0;
+            v[0] = warp_sum(((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7])));
+        }
+        (void)smem;
+    } else {
+        constexpr int RP = R <= 2 ? 2 : (R <= 4 ? 4 : 8), SH = RP == 2 ? 4 : (RP == 4 ? 3 : 2);  // lane >> SH: result
+        const int lane = tid & 31, warp = tid >> 5, nwarps = (nthreads + 31) >> 5;
+        double p[RP];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            double s = (tid < nwarps) ? smem[r][tid] : 0.0;
-            v[r] = warp_sum(s);
+        for (int r = 0; r < RP; ++r) p[r] = r < R ? v[r < R ? r : 0] : 0.0;
+        warp_sum_scatter<RP>(p);
+        if (!(lane & ((1 << SH) - 1)) && (lane >> SH) < R) smem[lane >> SH][warp] = p[0];
+        __syncthreads();
+        if (warp == 0) {
+#pragma unroll
+            for (int c = 0; c < R; c += 4) {  // eight lanes (the warps) a result, four results at a time
+                const int r = c + (lane >> 3), w = lane & 7;
+                double t = r < R && w < nwarps ? smem[r][w] : 0.0;
+                t += __shfl_xor_sync(0xffffffffu, t, 4);
+                t += __shfl_xor_sync(0xffffffffu, t, 2);
+                t += __shfl_xor_sync(0xffffffffu, t, 1);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const double tq = __shfl_sync(0xffffffffu, t, 8 * q);
+                    if (c + q < R) v[c + q < R ? c + q : 0] = tq;
+                }
+            }
         }
     }
     __syncthreads();
@@ -575,6 +597,7 @@ enum ScalarSlot : int {
     kSlotFdInvH = 20,     // RN(1/h) and RN(1/h^2) for the quotients
     kSlotFdInvHH = 21,
     kSlotPieceSums = 24,  // sums of squares of an evaluation's pieces, 8 entries
+    kSlotGmresRnorm = 56,  // 1 / ||w|| of the last Gram-Schmidt step
     kSlotGmresH = 64,      // Hessenberg column, m + 2 entries (m <= kMaxRestart)
     kSlotGmresH2 = 320,    // CGS2 second-pass coefficients, m + 1 entries
     kSlotGmresY = 640,     // least-squares solution y, m entries

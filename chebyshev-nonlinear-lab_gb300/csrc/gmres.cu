@@ -45,9 +45,15 @@ struct StoreAt {
     double* out;
     __device__ void operator()(const double (&t)[1]) const { *out = t[0]; }
 };
-struct StoreSqrtAt {
-    double* out;
-    __device__ void operator()(const double (&t)[1]) const { *out = __dsqrt_rn(t[0]); }
+// the norm and its reciprocal (0 for a zero vector): the division is done once, not by every thread of the pass
+// that normalises
+struct StoreNormAt {
+    double *out, *rout;
+    __device__ void operator()(const double (&t)[1]) const {
+        const double nrm = __dsqrt_rn(t[0]);
+        *out = nrm;
+        *rout = nrm > 0.0 ? __ddiv_rn(1.0, nrm) : 0.0;
+    }
 };
 
 // w -= hprev * Vprev (when Vprev is given); accumulate <w, Vcur> (or ||w||^2 when Vcur is null).
@@ -184,7 +190,7 @@ __global__ void __launch_bounds__(kRedThreads) k_icwy_dots(const double* __restr
 // terms of one are a chain.
 __global__ void __launch_bounds__(kRedThreads) k_icwy_update(double* __restrict__ w, const double* __restrict__ V,
                                                              size_t N, int j, const double* __restrict__ hcol,
-                                                             RedArgs red, double* norm) {
+                                                             RedArgs red, StoreNormAt fin) {
     pdl_wait();
     pdl_trigger();
     __shared__ double h[kIcwyMax];
@@ -211,16 +217,16 @@ __global__ void __launch_bounds__(kRedThreads) k_icwy_update(double* __restrict_
         }
     }
     block_sum<1>(s, sm);
-    grid_reduce_finish<1>(s, red, StoreSqrtAt{norm});
+    grid_reduce_finish<1>(s, red, fin);
 }
 
 // vnext = w / d with the norm d on the device, as k_div forms it (0 where d is not positive), so the host reads
-// the column after the kernel is launched.
-__global__ void k_div_dev(const double* __restrict__ w, const double* __restrict__ d, double* __restrict__ vnext,
-                          size_t N) {
+// the column after the kernel is launched.  rnorm: 1 / d where the step's finisher has formed it, or null.
+__global__ void k_div_dev(const double* __restrict__ w, const double* __restrict__ d, const double* __restrict__ rnorm,
+                          double* __restrict__ vnext, size_t N) {
     pdl_wait();
     pdl_trigger();
-    const double dv = *d, rd = dv > 0.0 ? __ddiv_rn(1.0, dv) : 0.0;
+    const double dv = *d, rd = rnorm ? *rnorm : (dv > 0.0 ? __ddiv_rn(1.0, dv) : 0.0);
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += stride)
         vnext[i] = dv > 0.0 ? w[i] * rd : 0.0;
@@ -750,7 +756,8 @@ void Gmres::arnoldi_mgs(size_t j, double* w) {
         launch_pdl(start ? k_icwy_dots<true> : k_icwy_dots<false>, dim3(gd, (unsigned)(j / 8 + 1 + start)), kRedThreads, 0,
                    ctx_.stream, (const double*)w, V, N, (int)j, ctx_.red, gram_.p, hcol);
         launch_pdl(k_icwy_update, (unsigned)std::min<size_t>(blocks, 8 * (size_t)ctx_.sm_count), kRedThreads, 0,
-                   ctx_.stream, w, V, N, (int)j, (const double*)hcol, ctx_.red, hcol + j + 1);
+                   ctx_.stream, w, V, N, (int)j, (const double*)hcol, ctx_.red,
+                   StoreNormAt{hcol + j + 1, ctx_.scalar(kSlotGmresRnorm)});
         ctx_.count_launch(2);
         ctx_.check_launch("arnoldi mgs");
         return;
@@ -762,8 +769,8 @@ void Gmres::arnoldi_mgs(size_t j, double* w) {
                                                               ctx_.red, StoreAt{hcol + i});
         ctx_.count_launch();
     }
-    launch_pdl(k_mgs<true, true, StoreSqrtAt>, g, kRedThreads, 0, ctx_.stream, w, V + j * N, hcol + j, nullptr, N, ctx_.red,
-                                                         StoreSqrtAt{hcol + j + 1});
+    launch_pdl(k_mgs<true, true, StoreNormAt>, g, kRedThreads, 0, ctx_.stream, w, V + j * N, hcol + j, nullptr, N, ctx_.red,
+                                                         StoreNormAt{hcol + j + 1, ctx_.scalar(kSlotGmresRnorm)});
     ctx_.count_launch();
     ctx_.check_launch("arnoldi mgs");
 }
@@ -1151,7 +1158,7 @@ GmresResult Gmres::solve(LinearOp& A, Precond* M, const double* b, double* x, co
                 arnoldi_mgs(j, w_.p);
             }
             launch_pdl(k_div_dev, eg, 256, 0, ctx_.stream, (const double*)w_.p, (const double*)(sl + j + 1),
-                       V_.p + (j + 1) * N, N);
+                       cgs1 || cgs2 ? nullptr : (const double*)ctx_.scalar(kSlotGmresRnorm), V_.p + (j + 1) * N, N);
             ctx_.count_launch();
             ctx_.fetch(sl, (int)(j + 2), col.data());
             if (cgs2) {
