@@ -187,7 +187,34 @@ __device__ __noinline__ void coarse_sweeps(int l, int sweeps, int order, bool al
     }
 }
 
-// r = b - h^-2 (6x - sum of neighbours [- c h^2 x]) at the slab's points
+// The 30 alternating sweeps of a coarsest level of 2^3 points (in CTA 0): lane p of warp 0 holds point p = 4i + 2j + k,
+// whose only neighbours are p ^ 4, p ^ 2 and p ^ 1 (i, j, k in that order; the absent ones would add +0.0).  Sixty
+// passes of the general form took 33 us a cycle, most of it indexing and FP64 additions of zeros.
+__device__ __noinline__ void coarse_sweeps2(int l) {
+    const CoarseLvl L = coarse_sh().cp.L[l];
+    double* base = coarse_base();
+    if (threadIdx.x < 32) {
+        const int p = threadIdx.x & 7, colour = __popc(p) & 1;
+        const double bs = base[L.offB + p] * L.inv;
+        double x = 0.0;
+#pragma unroll 1
+        for (int pass = 0; pass < 60; ++pass) {
+            const int c = (pass & 1) ^ ((pass >> 1) & 1);
+            double acc = bs;
+            acc = acc + __shfl_xor_sync(0xffffffffu, x, 4);
+            acc = acc + __shfl_xor_sync(0xffffffffu, x, 2);
+            acc = acc + __shfl_xor_sync(0xffffffffu, x, 1);
+            if (c == colour) x = div6(acc);
+        }
+        if (threadIdx.x < 8) {
+            const int P = ((1 + (p >> 2)) * L.m + 1 + ((p >> 1) & 1)) * L.m + 1 + (p & 1);
+            base[L.offX + (P & 1) * L.H + (P >> 1)] = x;
+        }
+    }
+    __syncthreads();
+}
+
+// r = b - h^-2 (6x - sum of neighbours) at the slab's points
 __device__ __noinline__ void coarse_residual(int l) {
     const CoarseShared& S = coarse_sh();
     const CoarseLvl L = S.cp.L[l];
@@ -384,6 +411,8 @@ __device__ __forceinline__ void coarse_cycle(const double* b_in, double* x_out) 
                 base[C.offX + (P & 1) * C.H + (P >> 1)] = div6(base[C.offB]) * C.inv;
             }
             __syncthreads();
+        } else if (C.n == 2) {
+            coarse_sweeps2(last);
         } else {
             coarse_sweeps(last, 30, 0, true, true);
         }

@@ -84,10 +84,12 @@ __device__ __forceinline__ float fma_t(float a, float b, float c) { return __fma
 // Coarse b = sum over the 27 fine points 2I+{0,1,2} of (w_a w_b w_c) r, weights (1/4,1/2,1/4),
 // summed a (i) outer, b (j), c (k) inner (poisson_mg.hpp:152-188).  Each weight product is a
 // power of two, so w*r is exact and the FMA equals the reference's multiply-then-add.  Also
-// stores bs = b * inv_c for the smoother.
-template <class T>
+// stores bs = b * inv_c for the smoother, and (FIRST_X) the coarse level's first smoothing pass, x = bs / 6 at the
+// colour-0 points.
+template <class T, bool FIRST_X = false>
 __global__ void __launch_bounds__(BX* BY) k_restrict(const T* __restrict__ rf, T* __restrict__ bc,
-                                                     T* __restrict__ bsc, int nf, int nc, double inv_c) {
+                                                     T* __restrict__ bsc, int nf, int nc, double inv_c,
+                                                     T* __restrict__ xc = nullptr) {
     pdl_wait();
     pdl_trigger();
     const int K = blockIdx.x * BX + threadIdx.x;
@@ -115,8 +117,10 @@ __global__ void __launch_bounds__(BX* BY) k_restrict(const T* __restrict__ rf, T
         }
     }
     const size_t q = ((size_t)I * nc + J) * nc + K;
+    const T bsv = acc * (T)inv_c;  // FP64: the reference's b * inv; FP32: RN32(b * RN32(inv))
     bc[q] = acc;
-    bsc[q] = acc * (T)inv_c;  // FP64: the reference's b * inv; FP32: RN32(b * RN32(inv))
+    bsc[q] = bsv;
+    if (FIRST_X && !((I + J + K) & 1)) xc[q] = div6(bsv);
 }
 
 // 1D interpolation stencil (poisson_mg.hpp:191-220).
@@ -166,6 +170,24 @@ __global__ void k_scale_in64(const double* __restrict__ r, double* __restrict__ 
     pdl_trigger();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < N; p += stride) bs[p] = r[p] * inv;
+}
+
+// The same with the cycle's first smoothing pass (colour 0 from x = 0: x = bs / 6), a pair of points {2kk, 2kk + 1} a
+// thread.
+__global__ void __launch_bounds__(BX* BY) k_scale_first64(const double* __restrict__ r, double* __restrict__ bs,
+                                                          double* __restrict__ x, int n,
+                                                          double inv) {
+    pdl_wait();
+    pdl_trigger();
+    const int k = 2 * (blockIdx.x * BX + threadIdx.x), j = blockIdx.y * BY + threadIdx.y, i = blockIdx.z;
+    if (j >= n || k >= n) return;
+    const size_t p = ((size_t)i * n + j) * n + k;
+    const bool two = k + 1 < n, odd = (i + j) & 1;  // the pair's second point has colour 0
+    const double s0 = r[p] * inv, s1 = two ? r[p + 1] * inv : 0.0;
+    bs[p] = s0;
+    if (two) bs[p + 1] = s1;
+    if (!odd) x[p] = div6(s0);
+    else if (two) x[p + 1] = div6(s1);
 }
 
 // b32 = RN32(r), bs32 = RN32(b32 * RN32(inv)) at the finest FP32 level (conversions in integer

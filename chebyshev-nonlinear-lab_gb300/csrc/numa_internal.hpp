@@ -402,6 +402,7 @@ private:
     template <class T> void cycle(size_t l);
     void cycle32(size_t l);
     bool first_fused32(size_t l) const;
+    bool first_fused64(size_t l) const;
     // FP32 cycle: levels from tail_l_ (n <= 15) down run in one CTA (k_mg_tail); SIZE_MAX = none.
     size_t tail_l_ = SIZE_MAX;
     size_t tail_smem_ = 0;

@@ -359,7 +359,9 @@ void PoissonMG::cycle(size_t l) {
     const dim3 blk(BX, BY);
     const dim3 cgrid(((n + 1) / 2 + BX - 1) / BX, (n + BY - 1) / BY, n);
 
+    const bool fused_first = first_fused64(l);
     auto pass = [&](int colour, bool first, bool outz) {
+        if (first && fused_first) return;  // already written by the producer of b
         if (first && outz) launch_pdl(k_rbgs<T, true, true>, cgrid, blk, 0, s, x, bs, z, n, colour);
         else if (first) launch_pdl(k_rbgs<T, true, false>, cgrid, blk, 0, s, x, bs, nullptr, n, colour);
         else if (outz) launch_pdl(k_rbgs<T, false, true>, cgrid, blk, 0, s, x, bs, z, n, colour);
@@ -398,7 +400,8 @@ void PoissonMG::cycle(size_t l) {
     const int nc = C.n;
     {
         const dim3 g((nc + BX - 1) / BX, (nc + BY - 1) / BY, nc);
-        launch_pdl(k_restrict<T>, g, blk, 0, s, r, bp<T>(C), bsp<T>(C), n, nc, C.inv);
+        launch_pdl(first_fused64(l + 1) ? k_restrict<T, true> : k_restrict<T>, g, blk, 0, s, (const T*)r, bp<T>(C), bsp<T>(C), n,
+                   nc, C.inv, xp<T>(C));
         ctx_.count_launch();
     }
     ctx_.check_launch("mg restrict");
@@ -418,6 +421,14 @@ void PoissonMG::cycle(size_t l) {
         ctx_.count_launch();
     }
     ctx_.check_launch("mg cycle");
+}
+
+// True when level l's first smoothing pass (colour 0 from x = 0) is fused into the producer of its right-hand side: one
+// launch a level fewer.
+bool PoissonMG::first_fused64(size_t l) const {
+    if (l == cl_l_) return false;
+    if (l + 1 == levels_.size()) return levels_[l]->n > 1;  // coarsest: 30 sweeps, the first from x = 0
+    return pre_ > 0;
 }
 
 // The FP32 cycle (precision extension): the same steps as cycle<double> in single precision.
@@ -521,7 +532,7 @@ void PoissonMG::cycle32(size_t l) {
     else if (csplit)
         launch_pdl(k_restrict_split<false>, rg2, blk, 0, s, r, C.b32.p, C.bs32.p, C.xs, n, nc, gc.half, (float)C.inv);
     else
-        launch_pdl(k_restrict<float>, rg, blk, 0, s, r, C.b32.p, C.bs32.p, n, nc, C.inv);
+        launch_pdl(k_restrict<float>, rg, blk, 0, s, (const float*)r, C.b32.p, C.bs32.p, n, nc, C.inv, (float*)nullptr);
     ctx_.count_launch();
     if (l == 0) coarse_cycle();
     else cycle32(l + 1);
@@ -589,7 +600,13 @@ void PoissonMG::apply(const double* r, double* z) {
             dev_copy(ctx_, r, alias_b_.p, N);
             b = alias_b_.p;
         }
-        launch_pdl(k_scale_in64, ew_grid(ctx_, N), 256, 0, ctx_.stream, b, L0.bs64.p, L0.inv, N);
+        if (first_fused64(0)) {
+            const int n = L0.n;
+            const dim3 g(((n + 1) / 2 + BX - 1) / BX, (n + BY - 1) / BY, n);
+            launch_pdl(k_scale_first64, g, dim3(BX, BY), 0, ctx_.stream, b, L0.bs64.p, z, n, L0.inv);
+        } else {
+            launch_pdl(k_scale_in64, ew_grid(ctx_, N), 256, 0, ctx_.stream, b, L0.bs64.p, L0.inv, N);
+        }
         ctx_.count_launch();
         x0_ = z;
         b0_ = b;
