@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(BX* BY, C32 ? 5 : 1) k_eval(const double* __re
                                                  float* __restrict__ f32_out, int n,
                                                  int ichunk, double lam, double h2inv, RedArgs red, double* norm_out,
                                                  int zoff, int norm_raw, const double2* __restrict__ lt2,
-                                                 const float2* __restrict__ ltf) {
+                                                 const float2* __restrict__ ltf, HostOut host) {
     pdl_wait();
     pdl_trigger();
     const int k = blockIdx.x * BX + threadIdx.x;
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(BX* BY, C32 ? 5 : 1) k_eval(const double* __re
         block_sum<1>(acc, sm);
         grid_reduce_finish<1>(acc, red, [norm_out, norm_raw] __device__(const double(&t)[1]) {
             *norm_out = norm_raw ? t[0] : __dsqrt_rn(t[0]);  // raw: a piece's sum of squares
-        });
+        }, host);
     }
 }
 
@@ -570,9 +570,10 @@ void Bratu3D::eval_launch(const double* x, double* out, double* c_out, double* n
     const RedArgs red = ctx_.red;
     const double2* t2 = lt_on_ ? lt2_.p : nullptr;
     const float2* tf = lt_on_ ? ltf_.p : nullptr;
+    const HostOut host = norm && !norm_raw ? ctx_.take(norm_out) : HostOut{};
     auto go = [&](auto kernel, double* c, float* c32v, float* f32v, double* nrm) {
         launch_pdl(kernel, grid, blk, 0, ctx_.stream, x, out, c, c32v, f32v, n, ichunk, lam, h2, red, nrm, zoff, norm_raw,
-                   t2, tf);
+                   t2, tf, host);
     };
     if (lt_on_) {
         if (c32 && norm) go(k_eval<true, true, true, true>, c_out, c32, f32, norm_out);

@@ -147,7 +147,8 @@ constexpr int kB2EvalRows = 32;  // rows a thread marches
 // instead of five FP64 instructions a species.
 template <bool NORM, bool FIXED = false>
 __global__ void __launch_bounds__(256) k_b2_eval(const double* __restrict__ w, const double* __restrict__ prev,
-                                                 double* __restrict__ out, B2Geom G, RedArgs red, double* norm_out) {
+                                                 double* __restrict__ out, B2Geom G, RedArgs red, double* norm_out,
+                                                 HostOut host) {
     pdl_wait();
     pdl_trigger();
     const int n = G.n;
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(256) k_b2_eval(const double* __restrict__ w, c
     if (NORM) {
         __shared__ double sm[1][32];
         block_sum<1>(acc, sm);
-        grid_reduce_finish<1>(acc, red, [norm_out] __device__(const double(&t)[1]) { *norm_out = __dsqrt_rn(t[0]); });
+        grid_reduce_finish<1>(acc, red, [norm_out] __device__(const double(&t)[1]) { *norm_out = __dsqrt_rn(t[0]); }, host);
     }
 }
 
@@ -988,11 +989,14 @@ void Brusselator2D::eval(const double* x, double* out, double*, double* norm_out
     if (grid.x * grid.y > (unsigned)kMaxRedBlocks) throw Status(NUMA_GPU_ERR_NOT_SUPPORTED, "Brusselator2D grid too large");
     const B2Geom G = b2_geom(n_, P_);
     if (norm_out && fixed_sum_)
-        launch_pdl(k_b2_eval<true, true>, grid, dim3(32, 8), 0, ctx_.stream, x, prev_.p, out, G, ctx_.red, norm_out);
+        launch_pdl(k_b2_eval<true, true>, grid, dim3(32, 8), 0, ctx_.stream, x, prev_.p, out, G, ctx_.red, norm_out,
+                   ctx_.take(norm_out));
     else if (norm_out)
-        launch_pdl(k_b2_eval<true>, grid, dim3(32, 8), 0, ctx_.stream, x, prev_.p, out, G, ctx_.red, norm_out);
+        launch_pdl(k_b2_eval<true>, grid, dim3(32, 8), 0, ctx_.stream, x, prev_.p, out, G, ctx_.red, norm_out,
+                   ctx_.take(norm_out));
     else  // an evaluation without the norm (the reference-facing F) keeps the FP64 differences
-        launch_pdl(k_b2_eval<false>, grid, dim3(32, 8), 0, ctx_.stream, x, prev_.p, out, G, ctx_.red, nullptr);
+        launch_pdl(k_b2_eval<false>, grid, dim3(32, 8), 0, ctx_.stream, x, prev_.p, out, G, ctx_.red, nullptr,
+                   HostOut{});
     ctx_.count_launch();
     ctx_.check_launch("Brusselator2D eval");
 }

@@ -54,6 +54,24 @@ struct RedArgs {
     unsigned* ticket;   // one counter, reset to 0 by the last block
 };
 
+// Where a reducing kernel leaves scalars for the waiting host: src[0..count) into mapped host memory, then the
+// sequence number behind them (dst null: nowhere).  src may hold earlier kernels' results beside this one's.
+struct HostOut {
+    double* dst = nullptr;
+    unsigned long long* word = nullptr;
+    unsigned long long seq = 0;
+    const double* src = nullptr;
+    int count = 0;
+};
+// Called by all threads of one block after the values are written (by any of them).
+__device__ __forceinline__ void host_publish(const HostOut& h, int tid, int nthreads) {
+    __syncthreads();
+    for (int i = tid; i < h.count; i += nthreads) h.dst[i] = __ldcg(h.src + i);
+    __threadfence_system();
+    __syncthreads();
+    if (tid == 0) asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(h.word), "l"(h.seq) : "memory");
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -130,8 +148,9 @@ __device__ __forceinline__ void block_sum(double (&v)[R], double (*smem)[32]) {
 
 // Publishes this block's totals and, in the last block to finish, reduces all partials and
 // calls fin(totals) on thread 0.  `v` must hold the block totals in thread 0 (block_sum output).
+// host: scalars to leave for the host once fin has run.
 template <int R, class Fin>
-__device__ __forceinline__ void grid_reduce_finish(const double (&v)[R], RedArgs red, Fin fin) {
+__device__ __forceinline__ void grid_reduce_finish(const double (&v)[R], RedArgs red, Fin fin, HostOut host = {}) {
     __shared__ bool am_last;
     __shared__ double tot_smem[R][32];
     const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
@@ -159,7 +178,9 @@ __device__ __forceinline__ void grid_reduce_finish(const double (&v)[R], RedArgs
     if (tid == 0) {
         fin(acc);
         *red.ticket = 0u;
+        if (host.dst) __threadfence();
     }
+    if (host.dst) host_publish(host, tid, nthreads);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -531,6 +552,16 @@ struct Context {
     Context& operator=(const Context&) = delete;
 
     void sync();
+    // Announces that src[0..count) will be fetched: the kernel whose reduction writes src[count - 1] takes the
+    // announcement (take) and leaves the values for the host itself, instead of a kernel of its own for that.
+    void expect(const double* src, int count);
+    HostOut take(const double* out) {
+        if (!armed.dst || out != armed.src + armed.count - 1) return {};
+        taken = true;
+        return armed;
+    }
+    HostOut armed;
+    bool taken = false;
     // Copies count device doubles to host memory and waits for them (and for all earlier work on the stream).
     void fetch(const double* dsrc, int count, double* host);
     double fetch1(const double* dsrc) {

@@ -60,7 +60,8 @@ struct StoreNormAt {
 template <bool HAS_PREV, bool NORM, class Fin>
 __global__ void __launch_bounds__(kRedThreads) k_mgs(double* __restrict__ w, const double* __restrict__ Vprev,
                                                      const double* __restrict__ hprev,
-                                                     const double* __restrict__ Vcur, size_t N, RedArgs red, Fin fin) {
+                                                     const double* __restrict__ Vcur, size_t N, RedArgs red, Fin fin,
+                                                     HostOut host = {}) {
     pdl_wait();
     pdl_trigger();
     __shared__ double sm[1][32];
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(kRedThreads) k_mgs(double* __restrict__ w, con
         s[0] = NORM ? __fma_rn(wi, wi, s[0]) : __fma_rn(wi, Vcur[i], s[0]);
     }
     block_sum<1>(s, sm);
-    grid_reduce_finish<1>(s, red, fin);
+    grid_reduce_finish<1>(s, red, fin, host);
 }
 
 // ---- modified Gram-Schmidt in the inverse compact WY form (see the head of the file)
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(kRedThreads) k_icwy_dots(const double* __restr
 // terms of one are a chain.
 __global__ void __launch_bounds__(kRedThreads) k_icwy_update(double* __restrict__ w, const double* __restrict__ V,
                                                              size_t N, int j, const double* __restrict__ hcol,
-                                                             RedArgs red, StoreNormAt fin) {
+                                                             RedArgs red, StoreNormAt fin, HostOut host) {
     pdl_wait();
     pdl_trigger();
     __shared__ double h[kIcwyMax];
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(kRedThreads) k_icwy_update(double* __restrict_
         }
     }
     block_sum<1>(s, sm);
-    grid_reduce_finish<1>(s, red, fin);
+    grid_reduce_finish<1>(s, red, fin, host);
 }
 
 // vnext = w / d with the norm d on the device, as k_div forms it (0 where d is not positive), so the host reads
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(kRedThreads) k_cgs(const double* w, const doub
                                                      const double* __restrict__ V, size_t ldv,
                                                      const double* __restrict__ hin, const double* __restrict__ sig2,
                                                      size_t N, RedArgs red, double* __restrict__ hout, double* wout,
-                                                     double* __restrict__ sig2_out) {
+                                                     double* __restrict__ sig2_out, HostOut host) {
     pdl_wait();
     pdl_trigger();
     constexpr int R = MODE == 2 ? 1 : CNT;
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(kRedThreads) k_cgs(const double* w, const doub
 #pragma unroll
                 for (int r = 0; r < R; ++r) hout[r] = t[r];
             }
-        });
+        }, host);
     }
 }
 
@@ -305,11 +306,12 @@ template <int MODE>
 void launch_cgs(Context& ctx, int cnt, const double* w, const double* v0, const double* V, size_t N,
                 const double* hin, const double* sig2, double* hout, double* wout, double* sig2_out) {
     const unsigned g = ctx.red_grid(N);
+    const HostOut host = MODE == 2 ? ctx.take(hout) : HostOut{};
     switch (cnt) {
 #define NUMA_CGS_CASE(K)                                                                                       \
     case K:                                                                                                    \
         launch_pdl(k_cgs<K, MODE>, g, kRedThreads, 0, ctx.stream, w, v0, V, N, hin, sig2, N, ctx.red, hout, wout,   \
-                                                          sig2_out);                                         \
+                   sig2_out, host);                                                                         \
         break;
         NUMA_CGS_CASE(1)
         NUMA_CGS_CASE(2)
@@ -449,7 +451,7 @@ __global__ void __launch_bounds__(kRedThreads) k_cgs_df(const float* w, const fl
                                                         const double* __restrict__ s2c,
                                                         const double* __restrict__ ascale, double* sig2, double* sig,
                                                         int j, size_t N, RedArgs red, double* __restrict__ hout,
-                                                        float* uout, float2* part_out) {
+                                                        float* uout, float2* part_out, HostOut host) {
     pdl_wait();
     pdl_trigger();
     constexpr int R = MODE == 2 ? 1 : CNT;
@@ -530,7 +532,7 @@ __global__ void __launch_bounds__(kRedThreads) k_cgs_df(const float* w, const fl
 #pragma unroll
                 for (int r = 0; r < R; ++r) hout[r] = t[r];
             }
-        });
+        }, host);
     }
 }
 
@@ -658,11 +660,12 @@ template <int MODE>
 void launch_cgs_df(Context& ctx, int cnt, const float* w, const float2* part_in, const float* u0, const float* U,
                    size_t N, const double* hin, const double* s2c, const double* ascale, double* sig2, double* sig,
                    int j, double* hout, float* uout, float2* part_out) {
+    const HostOut host = MODE == 2 ? ctx.take(hout) : HostOut{};
     switch (cnt) {
 #define NUMA_CGS_DF_CASE(K)                                                                                  \
     case K:                                                                                                  \
         launch_pdl(k_cgs_df<K, MODE>, cgs_grid<K, MODE>(ctx, N), kRedThreads, 0, ctx.stream, w, part_in, \
-                   u0, U, N, hin, s2c, ascale, sig2, sig, j, N, ctx.red, hout, uout, part_out);             \
+                   u0, U, N, hin, s2c, ascale, sig2, sig, j, N, ctx.red, hout, uout, part_out, host);       \
         break;
         NUMA_CGS_DF_CASE(1)
         NUMA_CGS_DF_CASE(2)
@@ -757,20 +760,20 @@ void Gmres::arnoldi_mgs(size_t j, double* w) {
                    ctx_.stream, (const double*)w, V, N, (int)j, ctx_.red, gram_.p, hcol);
         launch_pdl(k_icwy_update, (unsigned)std::min<size_t>(blocks, 8 * (size_t)ctx_.sm_count), kRedThreads, 0,
                    ctx_.stream, w, V, N, (int)j, (const double*)hcol, ctx_.red,
-                   StoreNormAt{hcol + j + 1, ctx_.scalar(kSlotGmresRnorm)});
+                   StoreNormAt{hcol + j + 1, ctx_.scalar(kSlotGmresRnorm)}, ctx_.take(hcol + j + 1));
         ctx_.count_launch(2);
         ctx_.check_launch("arnoldi mgs");
         return;
     }
-    launch_pdl(k_mgs<false, false, StoreAt>, g, kRedThreads, 0, ctx_.stream, w, nullptr, nullptr, V, N, ctx_.red, StoreAt{hcol});
+    launch_pdl(k_mgs<false, false, StoreAt>, g, kRedThreads, 0, ctx_.stream, w, nullptr, nullptr, V, N, ctx_.red, StoreAt{hcol}, HostOut{});
     ctx_.count_launch();
     for (size_t i = 1; i <= j; ++i) {
         launch_pdl(k_mgs<true, false, StoreAt>, g, kRedThreads, 0, ctx_.stream, w, V + (i - 1) * N, hcol + (i - 1), V + i * N, N,
-                                                              ctx_.red, StoreAt{hcol + i});
+                                                              ctx_.red, StoreAt{hcol + i}, HostOut{});
         ctx_.count_launch();
     }
     launch_pdl(k_mgs<true, true, StoreNormAt>, g, kRedThreads, 0, ctx_.stream, w, V + j * N, hcol + j, nullptr, N, ctx_.red,
-                                                         StoreNormAt{hcol + j + 1, ctx_.scalar(kSlotGmresRnorm)});
+                                                         StoreNormAt{hcol + j + 1, ctx_.scalar(kSlotGmresRnorm)}, ctx_.take(hcol + j + 1));
     ctx_.count_launch();
     ctx_.check_launch("arnoldi mgs");
 }
@@ -819,6 +822,7 @@ GmresResult Gmres::solve_lazy(LinearOp& A, Precond* M, const double* b, double* 
     double* sig2 = ctx_.scalar(kSlotGmresSig2);
     double bnorm = o.bnorm;
     if (bnorm < 0.0) {
+        ctx_.expect(sl, 1);
         dev_norm2(ctx_, b, N, sl);
         bnorm = ctx_.fetch1(sl);
     }
@@ -890,6 +894,7 @@ GmresResult Gmres::solve_lazy(LinearOp& A, Precond* M, const double* b, double* 
             v0 = r_init;
             given = false;
             first = false;
+            ctx_.expect(sl, 1);
             dev_norm2(ctx_, v0, N, sl);
             beta = ctx_.fetch1(sl);
         } else if (first) {
@@ -906,6 +911,7 @@ GmresResult Gmres::solve_lazy(LinearOp& A, Precond* M, const double* b, double* 
             launch_pdl(k_sub, eg, 256, 0, ctx_.stream, b, w_.p, r_.p, N);
             ctx_.count_launch();
             v0 = r_.p;
+            ctx_.expect(sl, 1);
             dev_norm2(ctx_, v0, N, sl);
             beta = ctx_.fetch1(sl);
         }
@@ -959,6 +965,7 @@ GmresResult Gmres::solve_lazy(LinearOp& A, Precond* M, const double* b, double* 
             }
             ++res.matvecs;
             const int cnt = (int)(j + 1);
+            ctx_.expect(sl, (int)(j + 2));
             float* unext = v32 ? V32_.p + (j + 1) * N : nullptr;
             if (v32 && !two_pass) {
                 cgs_dots_df(ctx_, cnt, W32_.p, u0, V32_.p, N, sl);
@@ -1073,6 +1080,7 @@ GmresResult Gmres::solve(LinearOp& A, Precond* M, const double* b, double* x, co
     if (save) save->clear();
 
     double* sl = ctx_.scalar(kSlotGmresH);
+    ctx_.expect(sl, 1);
     dev_norm2(ctx_, b, N, sl);
     const double bnorm = ctx_.fetch1(sl);
     if (bnorm == 0.0) {
@@ -1127,6 +1135,7 @@ GmresResult Gmres::solve(LinearOp& A, Precond* M, const double* b, double* x, co
             ctx_.count_launch();
             rv = r_.p;
         }
+        ctx_.expect(sl, 1);
         dev_norm2(ctx_, rv, N, sl);
         const double beta = ctx_.fetch1(sl);
         res.rel_res = beta / bnorm;
@@ -1150,6 +1159,7 @@ GmresResult Gmres::solve(LinearOp& A, Precond* M, const double* b, double* x, co
             ++res.precs;
             A.apply(zj, w_.p);
             ++res.matvecs;
+            ctx_.expect(sl, (int)(j + 2));
             if (cgs2) {
                 arnoldi_cgs2(j, w_.p);
             } else if (cgs1) {

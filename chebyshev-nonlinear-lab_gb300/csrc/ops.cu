@@ -89,7 +89,7 @@ __device__ __forceinline__ double bat(const double* __restrict__ a, int n, size_
 template <bool NORM>
 __global__ void __launch_bounds__(256) k_burgers_eval(const double* __restrict__ w, const double* __restrict__ g,
                                                       double* __restrict__ out, BurgersGeom G, RedArgs red,
-                                                      double* norm_out) {
+                                                      double* norm_out, HostOut host = {}) {
     const int j = blockIdx.x * 32 + threadIdx.x;
     const int i = blockIdx.y * 8 + threadIdx.y;
     const int n = G.n;
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) k_burgers_eval(const double* __restrict__
     if (NORM) {
         __shared__ double sm[1][32];
         block_sum<1>(acc, sm);
-        grid_reduce_finish<1>(acc, red, [norm_out] __device__(const double(&t)[1]) { *norm_out = __dsqrt_rn(t[0]); });
+        grid_reduce_finish<1>(acc, red, [norm_out] __device__(const double(&t)[1]) { *norm_out = __dsqrt_rn(t[0]); }, host);
     }
 }
 
@@ -257,7 +257,8 @@ void Burgers2D::eval(const double* x, double* out, double*, double* norm_out) {
     // the fused norm needs one partial per block; larger grids take the norm separately
     const bool fused = norm_out && (size_t)grid.x * grid.y <= (size_t)kMaxRedBlocks;
     if (fused)
-        k_burgers_eval<true><<<grid, dim3(32, 8), 0, ctx_.stream>>>(x, source_.p, out, G, ctx_.red, norm_out);
+        k_burgers_eval<true><<<grid, dim3(32, 8), 0, ctx_.stream>>>(x, source_.p, out, G, ctx_.red, norm_out,
+                                                                    ctx_.take(norm_out));
     else
         k_burgers_eval<false><<<grid, dim3(32, 8), 0, ctx_.stream>>>(x, source_.p, out, G, ctx_.red, nullptr);
     ctx_.count_launch();
