@@ -141,14 +141,13 @@ __device__ __forceinline__ double lap5(const double* __restrict__ a, int n, int 
 // forms its north difference N - c, keeping it as the next row's minus-south difference while the
 // thread marches down its rows.  Five FP64 instructions for each Laplacian instead of seven, the
 // same bits.  A warp covers 31 columns: lane 0 is the halo column whose east difference lane 1 needs.
-constexpr int kB2EvalRows = 32;  // rows a thread marches
 // FIXED (the mixed path's evaluation): each Laplacian as W + E + S + N - 4c in 64-bit fixed point, rounded
 // once (lap5_fixed, common.cuh; more accurate than the sum of rounded differences), on the integer pipe
 // instead of five FP64 instructions a species.
 template <bool NORM, bool FIXED = false>
 __global__ void __launch_bounds__(256) k_b2_eval(const double* __restrict__ w, const double* __restrict__ prev,
-                                                 double* __restrict__ out, B2Geom G, RedArgs red, double* norm_out,
-                                                 HostOut host) {
+                                                 double* __restrict__ out, B2Geom G, int rows, RedArgs red,
+                                                 double* norm_out, HostOut host) {
     pdl_wait();
     pdl_trigger();
     const int n = G.n;
@@ -160,7 +159,7 @@ __global__ void __launch_bounds__(256) k_b2_eval(const double* __restrict__ w, c
     const double* wu = w;
     const double* wv = w + nn;
     double acc[1] = {0.0};
-    const int i0 = ((int)blockIdx.y * 8 + (int)threadIdx.y) * kB2EvalRows, i1 = min(i0 + kB2EvalRows, n);
+    const int i0 = ((int)blockIdx.y * 8 + (int)threadIdx.y) * rows, i1 = min(i0 + rows, n);
     if (i0 < n) {
         const int im0 = i0 == 0 ? n - 1 : i0 - 1;
         double u = wu[(size_t)i0 * n + j], v = wv[(size_t)i0 * n + j];
@@ -217,8 +216,24 @@ __global__ void __launch_bounds__(256) k_b2_eval(const double* __restrict__ w, c
     }
 }
 
-dim3 b2_eval_grid(int n) {
-    return dim3((unsigned)((n + 30) / 31), (unsigned)((n + 8 * kB2EvalRows - 1) / (8 * kB2EvalRows)));
+// The rows a thread marches, and the grid.  Four blocks of this kernel fit an SM; the row chunks are chosen so that
+// the blocks fill whole waves of them: 32 rows always left 2048^2 with 3.5 blocks an SM (four on half of them: 147 us;
+// with 29 rows 139 us, the FP64 pipe) and 512^2 with 34 blocks in all.
+dim3 b2_eval_grid(int n, int sm_count, int& rows) {
+    const int kb = (n + 30) / 31, wave = 4 * sm_count, most = (n + 7) / 8;  // at least a row a thread
+    int best = 1;
+    double best_fill = 0.0;
+    for (int w = 1; w <= 4; ++w) {
+        const int chunks = std::max(1, std::min(w * wave / kb, most));
+        const int waves = (kb * chunks + wave - 1) / wave;
+        const double fill = (double)kb * chunks / ((double)waves * wave);
+        if (fill > best_fill + 0.01) {
+            best = chunks;
+            best_fill = fill;
+        }
+    }
+    rows = (n + 8 * best - 1) / (8 * best);
+    return dim3((unsigned)kb, (unsigned)((n + 8 * rows - 1) / (8 * rows)));
 }
 
 // J d with the point block [[c1 - 2uv, -u^2], [2uv - B, 1/dt + u^2]]:
@@ -985,17 +1000,19 @@ static B2Geom b2_geom(size_t n, const numa_brusselator2d_params& P) {
 void Brusselator2D::set_previous(const double* w) { dev_copy(ctx_, w, prev_.p, size()); }
 
 void Brusselator2D::eval(const double* x, double* out, double*, double* norm_out) {
-    const dim3 grid = b2_eval_grid((int)n_);
-    if (grid.x * grid.y > (unsigned)kMaxRedBlocks) throw Status(NUMA_GPU_ERR_NOT_SUPPORTED, "Brusselator2D grid too large");
+    int rows = 0;
+    const dim3 grid = b2_eval_grid((int)n_, ctx_.sm_count, rows);
+    if ((n_ + 30) / 31 * ((n_ + 255) / 256) > (size_t)kMaxRedBlocks)  // (the grid itself stays smaller)
+        throw Status(NUMA_GPU_ERR_NOT_SUPPORTED, "Brusselator2D grid too large");
     const B2Geom G = b2_geom(n_, P_);
     if (norm_out && fixed_sum_)
-        launch_pdl(k_b2_eval<true, true>, grid, dim3(32, 8), 0, ctx_.stream, x, prev_.p, out, G, ctx_.red, norm_out,
+        launch_pdl(k_b2_eval<true, true>, grid, dim3(32, 8), 0, ctx_.stream, x, prev_.p, out, G, rows, ctx_.red, norm_out,
                    ctx_.take(norm_out));
     else if (norm_out)
-        launch_pdl(k_b2_eval<true>, grid, dim3(32, 8), 0, ctx_.stream, x, prev_.p, out, G, ctx_.red, norm_out,
+        launch_pdl(k_b2_eval<true>, grid, dim3(32, 8), 0, ctx_.stream, x, prev_.p, out, G, rows, ctx_.red, norm_out,
                    ctx_.take(norm_out));
     else  // an evaluation without the norm (the reference-facing F) keeps the FP64 differences
-        launch_pdl(k_b2_eval<false>, grid, dim3(32, 8), 0, ctx_.stream, x, prev_.p, out, G, ctx_.red, nullptr,
+        launch_pdl(k_b2_eval<false>, grid, dim3(32, 8), 0, ctx_.stream, x, prev_.p, out, G, rows, ctx_.red, nullptr,
                    HostOut{});
     ctx_.count_launch();
     ctx_.check_launch("Brusselator2D eval");
