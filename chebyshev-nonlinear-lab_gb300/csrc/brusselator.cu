@@ -462,7 +462,8 @@ enum { kBPassNormal = 0, kBPassFirst = 1, kBPassLast = 2 };
 // of row i's points 2jj and 2jj + 1 (one of each colour) and updates the one of this colour; a warp
 // covers 32 consecutive points of one colour.
 //  Normal: x_c updated from the other colour.
-//  First (colour 0, x = 0 before the pass): x_0 = block^-1 b (neighbour sums are zeros), x_1 = 0;
+//  First (colour 0, x = 0 before the pass): x_0 = block^-1 b (neighbour sums are zeros); x_1 is left as it is,
+//    as the colour-1 pass that follows writes all of it and reads none;
 //    on the finest level the right-hand side is read from r (FP64 planes) and stored as b.
 //  Last (finest level, colour 0, the cycle's final pass): also writes z (FP64 planes) for both points,
 //    or, for an FP32 consumer, the same values as FP32 planes z32.
@@ -503,7 +504,6 @@ __global__ void __launch_bounds__(256) k_bmg_pass(T* __restrict__ X, T* __restri
     T u, v;
     block_update(load_blk(K, p), su, sv, su4, sv4, bu, bv, Su, Sv, u, v);
     st2(X, p, u, v);
-    if (MODE == kBPassFirst) st2(X, po, T(0), T(0));
     if (MODE == kBPassLast) {
         const auto o = ld2(X, po);
         if (z64) {
@@ -524,6 +524,11 @@ __global__ void __launch_bounds__(256) k_bmg_pass(T* __restrict__ X, T* __restri
 }
 
 // Residual r = b - (K x - diag(s) (S - 4x)) of one level at point (i, j).
+template <class T, class P>
+__device__ __forceinline__ void resid_value(const Blk<T>& k, P x, P bb, T Su, T Sv, T su, T sv, T& ru, T& rv) {
+    ru = bb.x - ((k.k11 * x.x + k.k12 * x.y) + su * (T(4) * x.x - Su));
+    rv = bb.y - ((k.k21 * x.x + k.k22 * x.y) + sv * (T(4) * x.y - Sv));
+}
 template <class T, bool SMEM_K = false>
 __device__ __forceinline__ void resid_at(const T* X, const T* Bv, const T* K, int n, int i, int j, T su, T sv, T& ru,
                                          T& rv) {
@@ -533,8 +538,7 @@ __device__ __forceinline__ void resid_at(const T* X, const T* Bv, const T* K, in
     const Blk<T> k = SMEM_K ? load_blk_s(K, p) : load_blk(K, p);
     T Su, Sv;
     nbr_sums(X, n, i, j, Su, Sv);
-    ru = bb.x - ((k.k11 * x.x + k.k12 * x.y) + su * (T(4) * x.x - Su));
-    rv = bb.y - ((k.k21 * x.x + k.k22 * x.y) + sv * (T(4) * x.y - Sv));
+    resid_value(k, x, bb, Su, Sv, su, sv, ru, rv);
 }
 
 // 9-point full weighting ((4c + 2((W + E) + (S + N))) + (((SW + SE) + NW) + NE)) / 16; S is row i-1.
@@ -546,7 +550,9 @@ __device__ __forceinline__ T fw9(T c, T w, T e, T s, T n, T sw, T se, T nw, T ne
 }
 
 // Residual of the finest-level points that a 16 x 16 tile of coarse points covers (33 x 33,
-// periodic), kept in shared memory, then full weighting into the coarse right-hand side.
+// periodic), kept in shared memory, then full weighting into the coarse right-hand side: FP64's restriction, bound
+// by the FP64 pipe (1.06 residuals formed a point; the march below forms 1.1 to 1.5: 278 us against 239 on 2048^2,
+// 20 against 12 on 128^2).
 template <class T>
 __global__ void __launch_bounds__(256) k_bmg_restrict(const T* __restrict__ X, const T* __restrict__ Bv,
                                                       const T* __restrict__ K, LvlArgs<T> L, T* __restrict__ Bc) {
@@ -574,22 +580,117 @@ __global__ void __launch_bounds__(256) k_bmg_restrict(const T* __restrict__ X, c
     st2(Bc, pidx(nc, I, J), fw(su_s), fw(sv_s));
 }
 
-// x_fine += bilinear periodic interpolation of x_coarse at the fine points (2I + {0,1}, 2J + {0,1}).
+// FP32's restriction: the residual of a level, full-weighted into the next level's right-hand side.  FIRST_X: also
+// that level's first smoothing pass (colour 0 from x = 0), where it is a launched level with a coarser one below: the
+// pass reads nothing but b and K of its own point, so its launch and its reading of b go.
+// Bound by L2 and HBM traffic (2048^2 FP32: x, b and K once are 134 MB).  A warp owns 31 coarse columns (lane 0 is
+// the column before them) and marches `rows` coarse rows: each step forms the residuals of the fine points
+// (2I + {0, 1}, 2J + {0, 1}) of its coarse point from 12 loaded pairs, takes those of the column before from the lane
+// to the left and those of the row before from its last step.  No shared memory and no barrier, and all of a step's
+// loads independent.  The tile
+// form's five rounds of points a block, with two integer divisions a point, took 34.2 us on 2048^2 and 10.0 on
+// 1024^2, and the pass after it 6.3 and 1.8: 33.0 and 7.2 for both.
+template <class T, bool FIRST_X>
+__global__ void __launch_bounds__(128) k_bmg_restrict_march(const T* __restrict__ X, const T* __restrict__ Bv,
+                                                            const T* __restrict__ K, LvlArgs<T> L, int rows,
+                                                            T* __restrict__ Bc, const T* __restrict__ Kc,
+                                                            T* __restrict__ Xc, LvlArgs<T> Lc) {
+    using P = typename P2<T>::t;
+    pdl_wait();
+    pdl_trigger();
+    const int nf = L.n, nc = nf / 2;
+    const int lane = threadIdx.x;
+    const int Jr = (int)blockIdx.x * 31 + lane - 1;
+    const int J = Jr < 0 ? nc - 1 : Jr < nc ? Jr : Jr - nc < nc ? Jr - nc : 0;  // lanes past the grid repeat columns
+    const bool owner = lane >= 1 && Jr < nc;
+    const int Jm = J == 0 ? nc - 1 : J - 1, Jp = J + 1 == nc ? 0 : J + 1;
+    const int I0 = ((int)blockIdx.y * 4 + (int)threadIdx.y) * rows, I1 = min(I0 + rows, nc);
+    if (I0 >= nc) return;  // whole warps
+    const T su = L.su, sv = L.sv;
+    // the colour halves of x, b and K, rows of nc points: (i, j) of colour 0 / 1 at i nc + j / 2
+    const size_t h = (size_t)nf * nc;
+    P p10, p11;  // the residuals of the row before: at (2I - 1, 2J) and (2I - 1, 2J + 1)
+    {
+        const int i = 2 * (I0 == 0 ? nc - 1 : I0 - 1) + 1;
+        resid_at(X, Bv, K, nf, i, 2 * J, su, sv, p10.x, p10.y);
+        resid_at(X, Bv, K, nf, i, 2 * J + 1, su, sv, p11.x, p11.y);
+    }
+    for (int I = I0; I < I1; ++I) {
+        const int im = I == 0 ? nf - 1 : 2 * I - 1, ip = I + 1 == nc ? 0 : 2 * I + 2;
+        const size_t q0 = (size_t)(2 * I) * nc, q1 = q0 + nc, qm = (size_t)im * nc + J, qp = (size_t)ip * nc + J;
+        const size_t q = pidx(nc, I, J);
+        const bool first = FIRST_X && ((I + J) & 1) == 0;
+        Blk<T> kc{};
+        if (first) kc = load_blk(Kc, q);
+        const auto x00 = ld2(X, q0 + J), x01 = ld2(X, h + q0 + J), x10 = ld2(X, h + q1 + J), x11 = ld2(X, q1 + J);
+        const auto w00 = ld2(X, h + q0 + Jm), w10 = ld2(X, q1 + Jm), e01 = ld2(X, q0 + Jp), e11 = ld2(X, h + q1 + Jp);
+        const auto s00 = ld2(X, h + qm), s01 = ld2(X, qm), n10 = ld2(X, qp), n11 = ld2(X, h + qp);
+        const auto b00 = ld2(Bv, q0 + J), b01 = ld2(Bv, h + q0 + J), b10 = ld2(Bv, h + q1 + J), b11 = ld2(Bv, q1 + J);
+        P r00, r01, r10, r11;
+        resid_value(load_blk(K, q0 + J), x00, b00, ((w00.x + x01.x) + s00.x) + x10.x,
+                    ((w00.y + x01.y) + s00.y) + x10.y, su, sv, r00.x, r00.y);
+        resid_value(load_blk(K, h + q0 + J), x01, b01, ((x00.x + e01.x) + s01.x) + x11.x,
+                    ((x00.y + e01.y) + s01.y) + x11.y, su, sv, r01.x, r01.y);
+        resid_value(load_blk(K, h + q1 + J), x10, b10, ((w10.x + x11.x) + x00.x) + n10.x,
+                    ((w10.y + x11.y) + x00.y) + n10.y, su, sv, r10.x, r10.y);
+        resid_value(load_blk(K, q1 + J), x11, b11, ((x10.x + e11.x) + x01.x) + n11.x,
+                    ((x10.y + e11.y) + x01.y) + n11.y, su, sv, r11.x, r11.y);
+        auto left = [](P a) {
+            a.x = __shfl_up_sync(0xffffffffu, a.x, 1);
+            a.y = __shfl_up_sync(0xffffffffu, a.y, 1);
+            return a;
+        };
+        const P w = left(r01), nw = left(r11), sw = left(p11);
+        const T bu = fw9(r00.x, w.x, r01.x, p10.x, r10.x, sw.x, p11.x, nw.x, r11.x);
+        const T bv = fw9(r00.y, w.y, r01.y, p10.y, r10.y, sw.y, p11.y, nw.y, r11.y);
+        if (owner) {
+            st2(Bc, q, bu, bv);
+            if (first) {
+                T u, v;
+                block_update(kc, Lc.su, Lc.sv, Lc.su4, Lc.sv4, bu, bv, T(0), T(0), u, v);
+                st2(Xc, q, u, v);
+            }
+        }
+        p10 = r10;
+        p11 = r11;
+    }
+}
+
+// The coarse rows a warp of k_bmg_restrict_march marches: as many (up to 8) as leave 24 warps an SM.
+int bmg_march_rows(int nc, int sm_count) {
+    const int most = (int)((size_t)nc * ((nc + 30) / 31) / ((size_t)sm_count * 24));
+    return std::max(1, std::min(8, most));
+}
+
+// The bilinear periodic interpolation of x_coarse at the fine point (2I + 1, 2J + 1), from the four coarse points
+// (I, J), (I + 1, J), (I, J + 1), (I + 1, J + 1).
+template <class P>
+__device__ __forceinline__ P interp11(P c00, P c10, P c01, P c11) {
+    using T = decltype(c00.x);
+    P r;
+    r.x = T(0.25) * (((c00.x + c10.x) + c01.x) + c11.x);
+    r.y = T(0.25) * (((c00.y + c10.y) + c01.y) + c11.y);
+    return r;
+}
+template <class P>
+__device__ __forceinline__ P add2(P a, P b) {
+    P r;
+    r.x = a.x + b.x;
+    r.y = a.y + b.y;
+    return r;
+}
+
+// x_fine += the interpolation of x_coarse at the fine points (2I, 2J) and (2I + 1, 2J + 1): those of colour 0.
+// The first post-smoothing pass writes every colour-1 point and reads none of them, so they take no correction.
 template <class T>
 __device__ __forceinline__ void prolong_point(const T* Xc, int nc, int I, int J, T* Xf) {
     const int I1 = I + 1 == nc ? 0 : I + 1, J1 = J + 1 == nc ? 0 : J + 1;
     const auto c00 = ld2(Xc, pidx(nc, I, J)), c10 = ld2(Xc, pidx(nc, I1, J));
     const auto c01 = ld2(Xc, pidx(nc, I, J1)), c11 = ld2(Xc, pidx(nc, I1, J1));
-    const int nf = 2 * nc;
-    const size_t f00 = pidx(nf, 2 * I, 2 * J), f10 = pidx(nf, 2 * I + 1, 2 * J);
-    const size_t f01 = pidx(nf, 2 * I, 2 * J + 1), f11 = pidx(nf, 2 * I + 1, 2 * J + 1);
-    // the four fine pairs are loaded before any is stored (the compiler cannot tell the addresses apart)
-    const auto x00 = ld2(Xf, f00), x10 = ld2(Xf, f10), x01 = ld2(Xf, f01), x11 = ld2(Xf, f11);
-    st2(Xf, f00, x00.x + c00.x, x00.y + c00.y);
-    st2(Xf, f10, x10.x + T(0.5) * (c00.x + c10.x), x10.y + T(0.5) * (c00.y + c10.y));
-    st2(Xf, f01, x01.x + T(0.5) * (c00.x + c01.x), x01.y + T(0.5) * (c00.y + c01.y));
-    st2(Xf, f11, x11.x + T(0.25) * (((c00.x + c10.x) + c01.x) + c11.x),
-        x11.y + T(0.25) * (((c00.y + c10.y) + c01.y) + c11.y));
+    const size_t f00 = (size_t)(2 * I) * nc + J, f11 = f00 + nc;
+    const auto x00 = add2(ld2(Xf, f00), c00), x11 = add2(ld2(Xf, f11), interp11(c00, c10, c01, c11));
+    st2(Xf, f00, x00.x, x00.y);
+    st2(Xf, f11, x11.x, x11.y);
 }
 
 template <class T>
@@ -600,6 +701,49 @@ __global__ void __launch_bounds__(256) k_bmg_prolong(const T* __restrict__ Xc, i
     const int I = blockIdx.y * 8 + threadIdx.y;
     if (I >= nc || J >= nc) return;
     prolong_point(Xc, nc, I, J, Xf);
+}
+
+// The prolongation and the first post-smoothing pass (colour 1) of a level in one kernel (FP32; in FP64 its
+// repeated interpolations and two serial block updates a thread cost more than the launch: 9.1 us against 3.1 + 3.6
+// on 128^2, 219 against 49 + 144 on 2048^2).  The pass reads the
+// corrected colour-0 points and writes the colour-1 points; the pass after it writes every colour-0 point and reads
+// none of them: the corrected values need not be stored at all.  Thread (x, y) owns coarse point (I, J) and updates
+// the fine points (2I, 2J + 1) and (2I + 1, 2J) from their six colour-0 neighbours, corrected from eight coarse
+// points as they are read.
+// Bound by L2 and HBM traffic, as the passes are; the prolongation by itself read and wrote all of x again, and
+// cost its launch on the smaller levels: 2048^2 12.1 + 13.2 us -> 19.8, 1024^2 2.7 + 3.5 -> 4.5.
+template <class T>
+__global__ void __launch_bounds__(256) k_bmg_prolong_pass(const T* __restrict__ Xc, T* __restrict__ X,
+                                                          const T* __restrict__ Bv, const T* __restrict__ K,
+                                                          LvlArgs<T> L) {
+    pdl_wait();
+    pdl_trigger();
+    const int nc = L.n / 2;
+    const int J = blockIdx.x * 32 + threadIdx.x;
+    const int I = blockIdx.y * 8 + threadIdx.y;
+    if (I >= nc || J >= nc) return;
+    const int Im = I == 0 ? nc - 1 : I - 1, Ip = I + 1 == nc ? 0 : I + 1;
+    const int Jm = J == 0 ? nc - 1 : J - 1, Jp = J + 1 == nc ? 0 : J + 1;
+    const auto c00 = ld2(Xc, pidx(nc, I, J)), c10 = ld2(Xc, pidx(nc, Ip, J));
+    const auto c01 = ld2(Xc, pidx(nc, I, Jp)), c11 = ld2(Xc, pidx(nc, Ip, Jp));
+    const auto cm0 = ld2(Xc, pidx(nc, Im, J)), cm1 = ld2(Xc, pidx(nc, Im, Jp));
+    const auto c0m = ld2(Xc, pidx(nc, I, Jm)), c1m = ld2(Xc, pidx(nc, Ip, Jm));
+    const size_t q0 = (size_t)(2 * I) * nc, q1 = q0 + nc;
+    // the corrected colour-0 points: own (0, 0) and (1, 1), (0, 0) of the cells after it in J and in I, (1, 1) of
+    // the cells before it in I and in J
+    const auto x00 = add2(ld2(X, q0 + J), c00), x11 = add2(ld2(X, q1 + J), interp11(c00, c10, c01, c11));
+    const auto xe = add2(ld2(X, q0 + Jp), c01), xn = add2(ld2(X, (size_t)(2 * Ip) * nc + J), c10);
+    const auto xs = add2(ld2(X, (size_t)(2 * Im + 1) * nc + J), interp11(cm0, c00, cm1, c01));
+    const auto xw = add2(ld2(X, q1 + Jm), interp11(c0m, c1m, c00, c10));
+    const size_t p01 = (size_t)L.n * nc + q0 + J, p10 = p01 + nc;
+    const auto b01 = ld2(Bv, p01), b10 = ld2(Bv, p10);
+    T u, v;
+    block_update(load_blk(K, p01), L.su, L.sv, L.su4, L.sv4, b01.x, b01.y, ((x00.x + xe.x) + xs.x) + x11.x,
+                 ((x00.y + xe.y) + xs.y) + x11.y, u, v);
+    st2(X, p01, u, v);
+    block_update(load_blk(K, p10), L.su, L.sv, L.su4, L.sv4, b10.x, b10.y, ((xw.x + x11.x) + x00.x) + xn.x,
+                 ((xw.y + x11.y) + x00.y) + xn.y, u, v);
+    st2(X, p10, u, v);
 }
 
 // The coarsest level in one block: x = 0, then `sweeps` red-black sweeps (colour 0, 1).
@@ -678,14 +822,13 @@ __global__ void __launch_bounds__(kBmgTailThreads<T>, 1) k_bmg_tail(const TailLv
         const T su = A.su, sv = A.sv, su4 = A.su4, sv4 = A.sv4;
         for (int idx = tid; idx < n * half; idx += nt) {
             const int i = idx / half, jj = idx - i * half;
-            const int j = 2 * jj + ((i + colour) & 1), jo = 2 * jj + 1 - ((i + colour) & 1);
+            const int j = 2 * jj + ((i + colour) & 1);
             const size_t p = pidx(n, i, j);
             const auto b = ld2(Bv, p);
             T Su = T(0), Sv = T(0), u, v;
             if (!first) nbr_sums(X, n, i, j, Su, Sv);
             block_update(load_blk_s(K, p), su, sv, su4, sv4, b.x, b.y, Su, Sv, u, v);
             st2(X, p, u, v);
-            if (first) st2(X, pidx(n, i, jo), T(0), T(0));
         }
         if (small) __syncwarp();
         else __syncthreads();
@@ -1175,6 +1318,12 @@ void BrussMG2D::set_state(const double* w) {
     ctx_.check_launch("BrussMG2D set_state");
 }
 
+// Whether level l's first smoothing pass is done by the restriction that forms its right-hand side.
+template <class T>
+bool BrussMG2D::first_fused(size_t l) const {
+    return sizeof(T) == 4 && l > 0 && (int)l != tail_first_ && l + 1 < levels_.size();
+}
+
 template <class T>
 void BrussMG2D::cycle(size_t l) {
     Level& L = *levels_[l];
@@ -1220,14 +1369,17 @@ void BrussMG2D::cycle(size_t l) {
         }
         return;
     }
-    // pre-smoothing: colours 0, 1; the first pass starts from x = 0
-    if (finest && r32_)
+    // pre-smoothing: colours 0, 1; the first pass starts from x = 0 (in FP32 the restriction that formed b
+    // has done it below the finest level)
+    if (finest && r32_) {
         launch_pdl(k_bmg_pass<T, kBPassFirst, float>, pgrid, blk, 0, s, X, Bv, K, A, 0, r32_, nullptr, nullptr);
-    else
-        launch_pdl(k_bmg_pass<T, kBPassFirst>, pgrid, blk, 0, s, X, Bv, K, A, 0, finest ? r0_ : nullptr, nullptr,
-                   nullptr);
+        ctx_.count_launch();
+    } else if (!first_fused<T>(l)) {
+        launch_pdl(k_bmg_pass<T, kBPassFirst>, pgrid, blk, 0, s, X, Bv, K, A, 0, finest ? r0_ : nullptr, nullptr, nullptr);
+        ctx_.count_launch();
+    }
     launch_pdl(k_bmg_pass<T, kBPassNormal>, pgrid, blk, 0, s, X, Bv, K, A, 1, nullptr, nullptr, nullptr);
-    ctx_.count_launch(2);
+    ctx_.count_launch();
     for (int k = 1; k < pre_; ++k) {
         launch_pdl(k_bmg_pass<T, kBPassNormal>, pgrid, blk, 0, s, X, Bv, K, A, 0, nullptr, nullptr, nullptr);
         launch_pdl(k_bmg_pass<T, kBPassNormal>, pgrid, blk, 0, s, X, Bv, K, A, 1, nullptr, nullptr, nullptr);
@@ -1235,16 +1387,40 @@ void BrussMG2D::cycle(size_t l) {
     }
     Level& C = *levels_[l + 1];
     const int nc = C.n;
-    launch_pdl(k_bmg_restrict<T>, dim3((unsigned)((nc + 15) / 16), (unsigned)((nc + 15) / 16)), dim3(16, 16), 0, s, 
-        X, Bv, K, A, tp<T>(C.b));
+    if constexpr (sizeof(T) == 4) {
+        const int rows = bmg_march_rows(nc, ctx_.sm_count);
+        const dim3 rgrid((unsigned)((nc + 30) / 31), (unsigned)((nc + 4 * rows - 1) / (4 * rows))), rblk(32, 4);
+        const LvlArgs<T> Ac{nc, (T)C.su, (T)C.sv, (T)(4.0 * C.su), (T)(4.0 * C.sv)};
+        if (first_fused<T>(l + 1))
+            launch_pdl(k_bmg_restrict_march<T, true>, rgrid, rblk, 0, s, X, Bv, K, A, rows, tp<T>(C.b), tp<T>(C.k),
+                       tp<T>(C.x), Ac);
+        else
+            launch_pdl(k_bmg_restrict_march<T, false>, rgrid, rblk, 0, s, X, Bv, K, A, rows, tp<T>(C.b), nullptr,
+                       nullptr, Ac);
+    } else {
+        launch_pdl(k_bmg_restrict<T>, dim3((unsigned)((nc + 15) / 16), (unsigned)((nc + 15) / 16)), dim3(16, 16), 0, s,
+                   X, Bv, K, A, tp<T>(C.b));
+    }
     ctx_.count_launch();
     if (finest) coarse_cycle();
     else cycle<T>(l + 1);
-    launch_pdl(k_bmg_prolong<T>, dim3((unsigned)((nc + 31) / 32), (unsigned)((nc + 7) / 8)), blk, 0, s, tp<T>(C.x), nc, X);
-    ctx_.count_launch();
+    const dim3 cgrid((unsigned)((nc + 31) / 32), (unsigned)((nc + 7) / 8));
+    constexpr bool fused_prolong = sizeof(T) == 4;
+    if constexpr (!fused_prolong) {
+        launch_pdl(k_bmg_prolong<T>, cgrid, blk, 0, s, tp<T>(C.x), nc, X);
+        ctx_.count_launch();
+    }
     // post-smoothing: colours 1, 0; the very last pass of the finest level writes z
     for (int k = 0; k < post_; ++k) {
-        launch_pdl(k_bmg_pass<T, kBPassNormal>, pgrid, blk, 0, s, X, Bv, K, A, 1, nullptr, nullptr, nullptr);
+        bool corrected = false;
+        if constexpr (fused_prolong) {
+            if (k == 0) {
+                launch_pdl(k_bmg_prolong_pass<T>, cgrid, blk, 0, s, tp<T>(C.x), X, Bv, K, A);
+                corrected = true;
+            }
+        }
+        if (!corrected)
+            launch_pdl(k_bmg_pass<T, kBPassNormal>, pgrid, blk, 0, s, X, Bv, K, A, 1, nullptr, nullptr, nullptr);
         if (finest && k + 1 == post_)
             launch_pdl(k_bmg_pass<T, kBPassLast>, pgrid, blk, 0, s, X, Bv, K, A, 0, nullptr, z0_, z32_);
         else

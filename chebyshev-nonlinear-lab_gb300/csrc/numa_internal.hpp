@@ -346,6 +346,8 @@ public:
     struct Level;
 
 private:
+    template <class T>
+    bool first_fused(size_t l) const;
     template <class T> void cycle(size_t l);
     void coarse_cycle();
     Context& ctx_;
