@@ -110,16 +110,16 @@ __global__ void __launch_bounds__(BX* BY) k_brestrict(MgPool F, MgPool C, const 
                                  blockIdx.x, blockIdx.y, blockIdx.z - q * zc);
 }
 
-// coarse pool grid q -> fine pool grid q, nc + 1 cell planes per grid
-template <bool ALL>
-__global__ void __launch_bounds__(BX* BY) k_bprolong(MgPool C, MgPool F, const int* __restrict__ act, int nc, int halfc,
-                                                     int nf, int halff) {
+// coarse pool grid q -> fine pool grid q with the first post-smoothing pass, nc + 1 cell planes per grid
+__global__ void __launch_bounds__(BX* BY) k_bprolong_pass(MgPool C, MgPool F, const int* __restrict__ act, int nc,
+                                                          int halfc, Split g) {
     pdl_wait();
     pdl_trigger();
     const int q = blockIdx.z / (nc + 1);
     if (!pool_active(F, act, q)) return;
-    prolong_split_body<true, ALL>(C.x + q * C.sx, F.x + q * F.sx, nc, halfc, nf, halff, blockIdx.x, blockIdx.y,
-                                  blockIdx.z - q * (nc + 1));
+    float* x = F.x + q * F.sx;
+    prolong_pass_split_body<true, 0>(C.x + q * C.sx, x, x + g.half, F.bs + q * F.sb + g.half, nc, halfc, g, blockIdx.x,
+                                     blockIdx.y, blockIdx.z - q * (nc + 1));
 }
 
 // 31^3 and below of every grid of the 31^3 pool: a cluster of 8 CTAs a grid (mg_chain.cuh).  The first top0 grids

@@ -802,15 +802,16 @@ void BatchSolver::Impl::vcycle(int j) {
         over_pool(0, P.K, nc + 1, [&](int a, int cnt) {
             MgPool Fw = V, Cw = CV;
             Fw.x += (long long)a * V.sx;
+            Fw.bs += (long long)a * V.sb;
             Fw.inst += a;
             Cw.x += (long long)a * CV.sx;
             Cw.inst += a;
             const dim3 cg((nc + 1 + BX - 1) / BX, (nc + 1 + BY - 1) / BY, cnt * (nc + 1));
-            launch_pdl(k_bprolong<false>, cg, blk, 0, s, Cw, Fw, act, nc, gc.half, n, g.half);
+            launch_pdl(k_bprolong_pass, cg, blk, 0, s, Cw, Fw, act, nc, gc.half, g);
             ctx.count_launch();
         });
         for (int sw = 0; sw < post; ++sw) {
-            pass(P, 0, P.K, kPassFull, 1, nullptr, 0);
+            if (sw > 0) pass(P, 0, P.K, kPassFull, 1, nullptr, 0);
             const bool last = sw + 1 == post;
             if (!last || P.cls < 0) {
                 pass(P, 0, P.K, kPassFull, 0, nullptr, 0);

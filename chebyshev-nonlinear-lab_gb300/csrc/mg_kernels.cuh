@@ -546,39 +546,18 @@ __device__ __forceinline__ void prolong_point(const float (&X)[2][2][2], const b
     *e = *e + acc;
 }
 
-// The same correction without the update: returns the weighted sum for fine point (A, B, C) of the cell.
-template <int A, int B, int C>
-__device__ __forceinline__ float prolong_sum(const float (&X)[2][2][2], const bool (&pi)[2], const bool (&pj)[2],
-                                             const bool (&pk)[2]) {
-    const float w = (A ? 1.0f : 0.5f) * (B ? 1.0f : 0.5f) * (C ? 1.0f : 0.5f);
-    float acc = 0.0f;
-#pragma unroll
-    for (int di = A; di < 2; ++di) {
-        if (!pi[di]) continue;
-#pragma unroll
-        for (int dj = B; dj < 2; ++dj) {
-            if (!pj[dj]) continue;
-#pragma unroll
-            for (int dk = C; dk < 2; ++dk) {
-                if (!pk[dk]) continue;
-                acc = __fmaf_rn(w, X[di][dj][dk], acc);
-            }
-        }
-    }
-    return acc;
-}
-
-// Fine x += trilinear interpolation of coarse x (k_prolong's arithmetic) on a split fine level.
-// A thread owns the coarse cell (I, J, K), I, J, K in [0, nc], i.e. the fine points
+// Fine x += trilinear interpolation of coarse x (k_prolong's arithmetic) on a split fine level: the cycles without
+// post-smoothing.  A thread owns the coarse cell (I, J, K), I, J, K in [0, nc], i.e. the fine points
 // (2I + a, 2J + b, 2K + c), a, b, c in {0, 1}, inside the grid; it loads the eight coarse values
-// around the cell once.  ALL = false: only the colour-0 fine points ((a + b + c) even), the only
-// ones the first post-smoothing pass reads.  The coarse level is split (odd nc) or natural.
-template <bool SPLIT_C, bool ALL>
-__device__ __forceinline__ void prolong_split_body(const float* __restrict__ xc, float* __restrict__ xf, int nc,
-                                                   int halfc, int nf, int halff, int bx, int by, int bz) {
-    const int K = bx * BX + threadIdx.x;
-    const int J = by * BY + threadIdx.y;
-    const int I = bz;
+// around the cell once.  The coarse level is split (odd nc) or natural.
+template <bool SPLIT_C>
+__global__ void __launch_bounds__(BX* BY) k_prolong_split(const float* __restrict__ xc, float* __restrict__ xf,
+                                                          int nc, int halfc, int nf, int halff) {
+    pdl_wait();
+    pdl_trigger();
+    const int K = blockIdx.x * BX + threadIdx.x;
+    const int J = blockIdx.y * BY + threadIdx.y;
+    const int I = blockIdx.z;
     if (K > nc || J > nc) return;
     const bool pi[2] = {I >= 1, I < nc}, pj[2] = {J >= 1, J < nc}, pk[2] = {K >= 1, K < nc};
     float X[2][2][2];
@@ -596,40 +575,136 @@ __device__ __forceinline__ void prolong_split_body(const float* __restrict__ xc,
                 X[di][dj][dk] = v;
             }
     const bool ia = I < nc, jb = J < nc, kc = K < nc;  // fine index 2I + 1 inside the grid
-    if (!ALL) {
-        // the four colour-0 points: their fine values are loaded before any is stored (the compiler
-        // cannot tell the four addresses apart, and would otherwise wait out each load in turn)
-        const int L0 = ((2 * I) * nf + 2 * J) * nf + 2 * K;
-        float* e0 = xf + split_at(L0, halff);
-        float* e1 = xf + split_at(L0 + nf + 1, halff);       // (0, 1, 1)
-        float* e2 = xf + split_at(L0 + nf * nf + 1, halff);  // (1, 0, 1)
-        float* e3 = xf + split_at(L0 + nf * nf + nf, halff); // (1, 1, 0)
-        const bool h1 = jb && kc, h2 = ia && kc, h3 = ia && jb;
-        const float v0 = *e0, v1 = h1 ? *e1 : 0.0f, v2 = h2 ? *e2 : 0.0f, v3 = h3 ? *e3 : 0.0f;
-        *e0 = v0 + prolong_sum<0, 0, 0>(X, pi, pj, pk);
-        if (h1) *e1 = v1 + prolong_sum<0, 1, 1>(X, pi, pj, pk);
-        if (h2) *e2 = v2 + prolong_sum<1, 0, 1>(X, pi, pj, pk);
-        if (h3) *e3 = v3 + prolong_sum<1, 1, 0>(X, pi, pj, pk);
-        return;
-    }
     prolong_point<0, 0, 0>(X, pi, pj, pk, xf, I, J, K, nf, halff);
     if (jb && kc) prolong_point<0, 1, 1>(X, pi, pj, pk, xf, I, J, K, nf, halff);
     if (ia && kc) prolong_point<1, 0, 1>(X, pi, pj, pk, xf, I, J, K, nf, halff);
     if (ia && jb) prolong_point<1, 1, 0>(X, pi, pj, pk, xf, I, J, K, nf, halff);
-    {
-        if (kc) prolong_point<0, 0, 1>(X, pi, pj, pk, xf, I, J, K, nf, halff);
-        if (jb) prolong_point<0, 1, 0>(X, pi, pj, pk, xf, I, J, K, nf, halff);
-        if (ia) prolong_point<1, 0, 0>(X, pi, pj, pk, xf, I, J, K, nf, halff);
-        if (ia && jb && kc) prolong_point<1, 1, 1>(X, pi, pj, pk, xf, I, J, K, nf, halff);
-    }
+    if (kc) prolong_point<0, 0, 1>(X, pi, pj, pk, xf, I, J, K, nf, halff);
+    if (jb) prolong_point<0, 1, 0>(X, pi, pj, pk, xf, I, J, K, nf, halff);
+    if (ia) prolong_point<1, 0, 0>(X, pi, pj, pk, xf, I, J, K, nf, halff);
+    if (ia && jb && kc) prolong_point<1, 1, 1>(X, pi, pj, pk, xf, I, J, K, nf, halff);
 }
 
-template <bool SPLIT_C, bool ALL>
-__global__ void __launch_bounds__(BX* BY) k_prolong_split(const float* __restrict__ xc, float* __restrict__ xf,
-                                                          int nc, int halfc, int nf, int halff) {
+// The prolongation (k_prolong's arithmetic) and the first post-smoothing pass (colour 1, k_rbgs<float>'s) of a split
+// level in one kernel.  The pass reads the corrected colour-0 points and writes every colour-1 point; the pass after
+// it writes every colour-0 point and reads none of them, so the corrected values are formed as they are read and
+// stored nowhere.  A thread owns the coarse cell (I, J, K), I, J, K in [0, nc], and updates its four colour-1 points
+// inside the grid, (2I + 1, 2J, 2K), (2I, 2J + 1, 2K), (2I, 2J, 2K + 1) and (2I + 1, 2J + 1, 2K + 1): of their 24
+// neighbours 16 are different points, corrected from 20 coarse values (absent ones are zeros, which leave the
+// interpolation's sums as they are).  x0, x1, bs1: the colour halves of x and the colour-1 half of b h^2.  NN > 0: the
+// grid size is a compile-time constant.  INNER: I and J have their neighbours on both sides, so that only the tests
+// on K remain.
+// Bound by the latency of its 40 loads a cell and their issue (245 instructions a cell).  The prolongation and the
+// pass by themselves: 255^3 19.5 + 19.7 us, 127^3 3.4 + 3.0, 63^3 1.3 + 1.3; together 35.5, 4.7 and 2.3.
+template <bool SPLIT_C, int NN, bool INNER>
+__device__ __forceinline__ void prolong_pass_split_cell(const float* __restrict__ xc, const float* __restrict__ x0,
+                                                        float* __restrict__ x1, const float* __restrict__ bs1, int nc,
+                                                        int halfc, const Split& g, int I, int J, int K) {
+    if (NN > 0) nc = (NN - 1) / 2;
+    const int n = NN > 0 ? NN : g.n;
+    const int hn = NN > 0 ? (NN - 1) / 2 : g.hn, hP = NN > 0 ? (NN * NN - 1) / 2 : g.hP, P = n * n;
+    // coarse I - 1, I, I + 1 exist (fine 2I - 1; 2I + 1, 2I + 2)
+    const bool im = INNER || I > 0, i1 = INNER || I < nc, i2 = INNER || I + 1 < nc;
+    const bool jm = INNER || J > 0, j1 = INNER || J < nc, j2 = INNER || J + 1 < nc;
+    const bool km = K > 0, k1 = K < nc, k2 = K + 1 < nc;
+    // x_coarse at (I + a, J + b, K + c), e = (a nc + b) nc + c points after the cell's: on a split level (nc odd, so
+    // e is even when a + b + c is) at e / 2 or (e - 1) / 2 after one of two fixed places
+    const int Lc0 = (I * nc + J) * nc + K;
+    const bool odd = Lc0 & 1;
+    const float* ce = SPLIT_C ? xc + (Lc0 >> 1) + (odd ? halfc : 0) : xc + Lc0;
+    const float* co = SPLIT_C ? xc + (Lc0 >> 1) + (odd ? 1 : halfc) : xc + Lc0;
+    auto coarse = [&](int a, int b, int c) {
+        const bool in = (a < 0 ? im : a ? i2 : i1) && (b < 0 ? jm : b ? j2 : j1) && (c < 0 ? km : c ? k2 : k1);
+        const int e = (a * nc + b) * nc + c;
+        if (!in) return 0.0f;
+        if (!SPLIT_C) return ce[e];
+        return ((a + b + c) & 1) ? co[(e - 1) >> 1] : ce[e >> 1];
+    };
+    float C[3][3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                if ((a == 2) + (b == 2) + (c == 2) < 2) C[a][b][c] = coarse(a - 1, b - 1, c - 1);
+    // x_0 at the fine point (2(I + a) + A, 2(J + b) + B, 2(K + c) + C), where `in` says that it is in the grid
+    const int m0 = (I * n + J) * n + K;
+    const float* xf = x0 + m0;
+    auto fine = [&](bool in, int off) { return in ? xf[off] : 0.0f; };
+    const int o011 = hn + 1, o101 = hP + 1, o110 = hP + hn + 1;
+    const float f000 = fine(true, 0), f011 = fine(j1 && k1, o011), f101 = fine(i1 && k1, o101), f110 = fine(i1 && j1, o110);
+    const float fi000 = fine(i1, P), fi011 = fine(i1 && j1 && k1, P + o011);
+    const float fj000 = fine(j1, n), fj101 = fine(i1 && j1 && k1, n + o101);
+    const float fk000 = fine(k1, 1), fk110 = fine(i1 && j1 && k1, 1 + o110);
+    const float gi110 = fine(im && j1, o110 - P), gi101 = fine(im && k1, o101 - P);
+    const float gj110 = fine(i1 && jm, o110 - n), gj011 = fine(jm && k1, o011 - n);
+    const float gk101 = fine(i1 && km, o101 - 1), gk011 = fine(j1 && km, o011 - 1);
+    const float b100 = i1 ? bs1[m0 + hP] : 0.0f, b010 = j1 ? bs1[m0 + hn] : 0.0f, b001 = k1 ? bs1[m0] : 0.0f;
+    const float b111 = i1 && j1 && k1 ? bs1[m0 + o110] : 0.0f;
+    // the corrections of the points (0, 0, 0), (0, 1, 1), (1, 0, 1), (1, 1, 0) of cell (I + a, J + b, K + c)
+    auto s000 = [&](int a, int b, int c) {
+        float acc = 0.0f;
+#pragma unroll
+        for (int di = 0; di < 2; ++di)
+#pragma unroll
+            for (int dj = 0; dj < 2; ++dj)
+#pragma unroll
+                for (int dk = 0; dk < 2; ++dk) acc = __fmaf_rn(0.125f, C[a + di][b + dj][c + dk], acc);
+        return acc;
+    };
+    auto two = [](float p, float q) { return __fmaf_rn(0.5f, q, __fmaf_rn(0.5f, p, 0.0f)); };
+    auto s011 = [&](int a, int b, int c) { return two(C[a][b + 1][c + 1], C[a + 1][b + 1][c + 1]); };
+    auto s101 = [&](int a, int b, int c) { return two(C[a + 1][b][c + 1], C[a + 1][b + 1][c + 1]); };
+    auto s110 = [&](int a, int b, int c) { return two(C[a + 1][b + 1][c], C[a + 1][b + 1][c + 1]); };
+    const float v000 = f000 + s000(0, 0, 0), v011 = f011 + s011(0, 0, 0), v101 = f101 + s101(0, 0, 0),
+                v110 = f110 + s110(0, 0, 0);
+    auto update = [](float b, float a0, float a1, float a2, float a3, float a4, float a5) {
+        float acc = b;
+        acc = acc + a0;
+        acc = acc + a1;
+        acc = acc + a2;
+        acc = acc + a3;
+        acc = acc + a4;
+        acc = acc + a5;
+        return div6(acc);
+    };
+    // a neighbour outside the grid counts as +0 (those that a stored point always has are not tested)
+    if (i1)
+        x1[m0 + hP] = update(b100, v000, fi000 + s000(1, 0, 0), jm ? gj110 + s110(0, -1, 0) : 0.0f, j1 ? v110 : 0.0f,
+                             km ? gk101 + s101(0, 0, -1) : 0.0f, k1 ? v101 : 0.0f);
+    if (j1)
+        x1[m0 + hn] = update(b010, im ? gi110 + s110(-1, 0, 0) : 0.0f, i1 ? v110 : 0.0f, v000, fj000 + s000(0, 1, 0),
+                             km ? gk011 + s011(0, 0, -1) : 0.0f, k1 ? v011 : 0.0f);
+    if (k1)
+        x1[m0] = update(b001, im ? gi101 + s101(-1, 0, 0) : 0.0f, i1 ? v101 : 0.0f, jm ? gj011 + s011(0, -1, 0) : 0.0f,
+                        j1 ? v011 : 0.0f, v000, fk000 + s000(0, 0, 1));
+    if (i1 && j1 && k1)
+        x1[m0 + o110] = update(b111, v011, fi011 + s011(1, 0, 0), v101, fj101 + s101(0, 1, 0), v110,
+                               fk110 + s110(0, 0, 1));
+}
+
+template <bool SPLIT_C, int NN>
+__device__ __forceinline__ void prolong_pass_split_body(const float* __restrict__ xc, const float* __restrict__ x0,
+                                                        float* __restrict__ x1, const float* __restrict__ bs1, int nc,
+                                                        int halfc, const Split& g, int bx, int by, int bz) {
+    const int K = bx * BX + threadIdx.x;
+    const int J = by * BY + threadIdx.y;  // one of each a warp
+    const int I = bz;
+    if (K > nc || J > nc) return;
+    if (I > 0 && I + 1 < nc && J > 0 && J + 1 < nc)
+        prolong_pass_split_cell<SPLIT_C, NN, true>(xc, x0, x1, bs1, nc, halfc, g, I, J, K);
+    else
+        prolong_pass_split_cell<SPLIT_C, NN, false>(xc, x0, x1, bs1, nc, halfc, g, I, J, K);
+}
+
+template <bool SPLIT_C, int NN>
+__global__ void __launch_bounds__(BX* BY) k_prolong_pass_split(const float* __restrict__ xc, float* __restrict__ x,
+                                                               const float* __restrict__ bs, int nc, int halfc,
+                                                               Split g) {
     pdl_wait();
     pdl_trigger();
-    prolong_split_body<SPLIT_C, ALL>(xc, xf, nc, halfc, nf, halff, blockIdx.x, blockIdx.y, blockIdx.z);
+    prolong_pass_split_body<SPLIT_C, NN>(xc, x, x + g.half, bs + g.half, nc, halfc, g, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // b32 = RN32(r), bs32 = RN32(b32 * inv) into the split layout at the finest level; WRITE_X: also

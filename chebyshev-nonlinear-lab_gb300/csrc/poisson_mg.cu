@@ -537,15 +537,20 @@ void PoissonMG::cycle32(size_t l) {
     if (l == 0) coarse_cycle();
     else cycle32(l + 1);
     const dim3 cg((nc + 1 + BX - 1) / BX, (nc + 1 + BY - 1) / BY, nc + 1);
-    if (post_ > 0) {
-        if (csplit) launch_pdl(k_prolong_split<true, false>, cg, blk, 0, s, C.cur32, x, nc, gc.half, n, g.half);
-        else launch_pdl(k_prolong_split<false, false>, cg, blk, 0, s, C.cur32, x, nc, gc.half, n, g.half);
+    if (post_ > 0) {  // with the first post-smoothing pass
+        if (!csplit) launch_pdl(k_prolong_pass_split<false, 0>, cg, blk, 0, s, C.cur32, x, bs, nc, gc.half, g);
+        else if (n == 255) launch_pdl(k_prolong_pass_split<true, 255>, cg, blk, 0, s, C.cur32, x, bs, nc, gc.half, g);
+        else if (n == 127) launch_pdl(k_prolong_pass_split<true, 127>, cg, blk, 0, s, C.cur32, x, bs, nc, gc.half, g);
+        else launch_pdl(k_prolong_pass_split<true, 0>, cg, blk, 0, s, C.cur32, x, bs, nc, gc.half, g);
     } else {
-        if (csplit) launch_pdl(k_prolong_split<true, true>, cg, blk, 0, s, C.cur32, x, nc, gc.half, n, g.half);
-        else launch_pdl(k_prolong_split<false, true>, cg, blk, 0, s, C.cur32, x, nc, gc.half, n, g.half);
+        if (csplit) launch_pdl(k_prolong_split<true>, cg, blk, 0, s, C.cur32, x, nc, gc.half, n, g.half);
+        else launch_pdl(k_prolong_split<false>, cg, blk, 0, s, C.cur32, x, nc, gc.half, n, g.half);
     }
     ctx_.count_launch();
-    for (int sw = 0; sw < post_; ++sw) sweep(1, false, sw == post_ - 1);
+    for (int sw = 0; sw < post_; ++sw) {
+        if (sw > 0) pass(1, false, false);
+        pass(0, false, sw == post_ - 1);
+    }
     if (z && post_ == 0) out_z();
     ctx_.check_launch("mg cycle (fp32)");
 }
