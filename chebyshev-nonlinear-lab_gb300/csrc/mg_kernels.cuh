@@ -518,6 +518,165 @@ __global__ void __launch_bounds__(BX* BY) k_restrict_split(const float* __restri
     restrict_split_body<FIRST_X>(rf, bc, bsc, xc, nf, nc, halfc, inv_c, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
+// Residual and restriction of a split level over an odd (hence split) coarse one, in one kernel: the residual is
+// never stored.  A block owns the coarse points of kRrRows rows J and blockDim.x - 1 columns K, and marches over the
+// fine planes of `depth` coarse planes.  Thread (tx, ty) forms the residuals at its fine rows 2J, 2J + 1 and columns
+// 2K, 2K + 1 of each plane (residual_pair's order of subtractions), keeping x of the planes before and after in
+// registers; the last lane and the last row of threads form those that only the restriction of their neighbours
+// needs.  The values cross between threads through shared memory, and each plane's nine are added to the two coarse
+// points in flight in k_restrict's order (the planes follow in its order).  FIRST_X: also the coarse level's first
+// smoothing pass, x = bs / 6 at colour 0.  BNAT: as residual_split_body.
+// Bound by the latency of a plane's 16 loads and its barrier, with 32 warps an SM: 46.5 us on 255^3 (62 before the
+// loads from memory were issued a plane ahead; with three rows a block 47.6), 6.2 on 127^3 and 3.4 on 63^3.  The
+// residual and the restriction as two kernels, with the residual written and read again: 44.0 + 18.8, 5.4 + 3.0 and
+// 2.0 + 1.8 us.
+constexpr int kRrRows = 7, kRrMaxCols = 128, kRrThreads = 1024;  // threads an SM (64 registers each)
+
+template <int NN, bool BNAT, bool FIRST_X>
+__device__ __forceinline__ void residual_restrict_body(const float* __restrict__ x, const float* __restrict__ b,
+                                                       float* __restrict__ bc, float* __restrict__ bsc,
+                                                       float* __restrict__ xc, const Split& g, int nc, int halfc,
+                                                       float h2inv, float inv_c, int depth, int bx, int by, int bz) {
+    __shared__ float2 sa[2][kRrRows + 1][kRrMaxCols];  // residuals at (2J, 2K), (2J, 2K + 1)
+    __shared__ float2 sb[2][kRrRows][kRrMaxCols];      // at (2J + 1, 2K), (2J + 1, 2K + 1)
+    if (NN > 0) nc = (NN - 1) / 2;
+    const int n = NN > 0 ? NN : g.n, P = n * n;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int Kr = bx * ((int)blockDim.x - 1) + tx, Jr = by * kRrRows + ty;
+    const bool own = tx + 1 < (int)blockDim.x && Kr < nc && ty < kRrRows && Jr < nc;
+    const int K = min(Kr, nc), J = min(Jr, nc);  // threads past the grid repeat its last column or row
+    const bool colB = K < nc, rowB = J < nc, jlo = J > 0, klo = K > 0;
+    const int I0 = bz * depth, I1 = min(I0 + depth, nc);
+    // The even natural index of (2I, 2J, 2K) and, from it, the point (2I + a, 2J + r, 2K + k): e = a n^2 + r n + k
+    // points on, of colour e & 1 = (a + r + k) & 1 (n odd), at e / 2 or (e - 1) / 2 after the same place of its half.
+    const int L0 = (2 * I0 * n + 2 * J) * n + 2 * K;
+    const float* x0 = x + (L0 >> 1);
+    const float* x1 = x0 + g.half;
+    const float* b0 = BNAT ? b + L0 : b + (L0 >> 1);
+    const float* b1 = b0 + g.half;
+    auto at = [&](const float* v0, const float* v1, int a, int r, int k) {
+        const int e = a * P + r * n + k;
+        return ((a + r + k) & 1) ? v1[(e - 1) >> 1] : v0[e >> 1];
+    };
+    auto xat = [&](int a, int r, int k) { return at(x0, x1, a, r, k); };
+    auto bat = [&](int a, int r, int k) { return BNAT ? b0[a * P + r * n + k] : at(b0, b1, a, r, k); };
+    float pAa = 0.0f, pAb = 0.0f, pBa = 0.0f, pBb = 0.0f;  // x of plane i - 1: rows 2J (A), 2J + 1 (B); columns 2K, 2K + 1
+    if (I0 > 0) pAa = xat(-1, 0, 0), pAb = xat(-1, 0, 1), pBa = xat(-1, 1, 0), pBb = xat(-1, 1, 1);
+    float cAa = xat(0, 0, 0), cAb = xat(0, 0, 1), cBa = xat(0, 1, 0), cBb = xat(0, 1, 1);
+    float nAa = 0.0f, nAb = 0.0f, nBa = 0.0f, nBb = 0.0f;  // plane i + 1
+    if (I0 < nc) nAa = xat(1, 0, 0), nAb = xat(1, 0, 1), nBa = xat(1, 1, 0), nBb = xat(1, 1, 1);
+    float bAa, bAb, bBa, bBb;  // b of plane i
+    auto load_b = [&](int a) {
+        bAa = bat(a, 0, 0), bAb = colB ? bat(a, 0, 1) : 0.0f;
+        bBa = rowB ? bat(a, 1, 0) : 0.0f, bBb = rowB && colB ? bat(a, 1, 1) : 0.0f;
+    };
+    load_b(0);
+    float acc = 0.0f;
+    float v[9];  // the plane's residuals at rows 2J .. 2J + 2, columns 2K .. 2K + 2
+    // plane 2I + a (a a constant, 0 or 1); x of the plane after the next and b of the next, which come from memory, are
+    // loaded a plane ahead.  more, more2: there is a plane after it, and one after that
+    auto plane = [&](int a, bool more, bool more2) {
+        float mAa = 0.0f, mAb = 0.0f, mBa = 0.0f, mBb = 0.0f;
+        if (more2) mAa = xat(a + 2, 0, 0), mAb = xat(a + 2, 0, 1), mBa = xat(a + 2, 1, 0), mBb = xat(a + 2, 1, 1);
+        const float qAa = bAa, qAb = bAb, qBa = bBa, qBb = bBb;
+        if (more) load_b(a + 1);
+        const float sAa = jlo ? xat(a, -1, 0) : 0.0f, sAb = jlo ? xat(a, -1, 1) : 0.0f;
+        const float tBa = xat(a, 2, 0), tBb = xat(a, 2, 1);
+        const float lA = klo ? xat(a, 0, -1) : 0.0f, lB = klo ? xat(a, 1, -1) : 0.0f;
+        const float rA = xat(a, 0, 2), rB = xat(a, 1, 2);
+        auto resid = [h2inv](float bv, float xv, float im, float ip, float jm, float jp, float km, float kp) {
+            float t = 6.0f * xv;
+            t = t - im;
+            t = t - ip;
+            t = t - jm;
+            t = t - jp;
+            t = t - km;
+            t = t - kp;
+            return bv - h2inv * t;
+        };
+        v[0] = resid(qAa, cAa, pAa, nAa, sAa, rowB ? cBa : 0.0f, lA, colB ? cAb : 0.0f);
+        v[1] = resid(qAb, cAb, pAb, nAb, sAb, rowB ? cBb : 0.0f, cAa, rA);
+        sa[a][ty][tx] = make_float2(v[0], v[1]);
+        if (ty < kRrRows) {
+            v[3] = resid(qBa, cBa, pBa, nBa, cAa, tBa, lB, colB ? cBb : 0.0f);
+            v[4] = resid(qBb, cBb, pBb, nBb, cAb, tBb, cBa, rB);
+            sb[a][ty][tx] = make_float2(v[3], v[4]);
+        }
+        __syncthreads();
+        if (own) {
+            v[2] = sa[a][ty][tx + 1].x;
+            v[5] = sb[a][ty][tx + 1].x;
+            const float2 t2 = sa[a][ty + 1][tx];
+            v[6] = t2.x;
+            v[7] = t2.y;
+            v[8] = sa[a][ty + 1][tx + 1].x;
+        }
+        pAa = cAa, pAb = cAb, pBa = cBa, pBb = cBb;
+        cAa = nAa, cAb = nAb, cBa = nBa, cBb = nBb;
+        nAa = mAa, nAb = mAb, nBa = mBa, nBb = mBb;
+    };
+    auto add = [&](int a, float s) {
+        const float w[3] = {0.25f, 0.5f, 0.25f};
+#pragma unroll
+        for (int q = 0; q < 9; ++q) s = __fmaf_rn(w[a] * w[q / 3] * w[q % 3], v[q], s);
+        return s;
+    };
+    for (int I = I0;; ++I) {
+        plane(0, I < I1, I < nc);
+        if (own && I > I0) {  // the last plane of coarse plane I - 1
+            acc = add(2, acc);
+            const int Lc = ((I - 1) * nc + J) * nc + K;
+            const int q = split_at(Lc, halfc);
+            const float bsv = acc * inv_c;
+            bc[q] = acc;
+            bsc[q] = bsv;
+            if (FIRST_X && !(Lc & 1)) xc[q] = div6(bsv);
+        }
+        if (I == I1) break;
+        acc = add(0, 0.0f);
+        plane(1, true, I + 1 < nc);
+        acc = add(1, acc);
+        x0 += P;
+        x1 += P;
+        b0 += BNAT ? 2 * P : P;
+        b1 += P;
+    }
+}
+
+template <int NN, bool BNAT, bool FIRST_X>
+__global__ void __launch_bounds__(kRrMaxCols*(kRrRows + 1), kRrThreads / (kRrMaxCols * (kRrRows + 1))) k_residual_restrict(
+    const float* __restrict__ x, const float* __restrict__ b, float* __restrict__ bc, float* __restrict__ bsc,
+    float* __restrict__ xc, Split g, int nc, int halfc, float h2inv, float inv_c, int depth) {
+    pdl_wait();
+    pdl_trigger();
+    residual_restrict_body<NN, BNAT, FIRST_X>(x, b, bc, bsc, xc, g, nc, halfc, h2inv, inv_c, depth, blockIdx.x,
+                                              blockIdx.y, blockIdx.z);
+}
+
+// Whether a level's cells fill the lanes of residual_restrict's rows (7 of 8 at least): where they do not (95^3: 48 of
+// 64) the two kernels are faster, 93.3 us for the V-cycle against 96.6.
+inline bool rr_fits(int nc) {
+    const int cols = std::min((nc + 1 + 31) / 32 * 32, kRrMaxCols);
+    const int tiles_k = (nc + cols - 2) / (cols - 1);
+    return 8 * (nc + 1) >= 7 * tiles_k * cols;
+}
+
+// The shape of a residual_restrict launch: columns for the nc + 1 cells of a row where 128 reach, and the coarse
+// planes a block marches such that all blocks (kRrThreads an SM) run at once, if there are that many.
+struct RrShape {
+    dim3 grid, block;
+    int depth;
+};
+inline RrShape rr_shape(int nc, int sm_count) {
+    const int cols = std::min((nc + 1 + 31) / 32 * 32, kRrMaxCols);
+    const int tiles_k = (nc + cols - 2) / (cols - 1), tiles_j = (nc + kRrRows - 1) / kRrRows;
+    const int resident = sm_count * (kRrThreads / (cols * (kRrRows + 1)));
+    const int chunks = std::max(1, std::min(nc, (int)((long long)resident / ((long long)tiles_k * tiles_j))));
+    const int depth = (nc + chunks - 1) / chunks;
+    return RrShape{dim3((unsigned)tiles_k, (unsigned)tiles_j, (unsigned)((nc + depth - 1) / depth)),
+                   dim3((unsigned)cols, kRrRows + 1), depth};
+}
+
 // One fine point of a prolongation cell: x_f += sum over the present coarse neighbours (in the
 // order i, j, k of k_prolong) of w * X, with w = (A ? 1 : 1/2)(B ? 1 : 1/2)(C ? 1 : 1/2).
 // X[di][dj][dk] holds the coarse values at (I - 1 + di, J - 1 + dj, K - 1 + dk); pr*[d] tells

@@ -515,25 +515,40 @@ void PoissonMG::cycle32(size_t l) {
     Level& C = *levels_[l + 1];
     const int nc = C.n;
     const bool csplit = (nc & 1) != 0;
-    {
+    const Split gc = make_split(nc);
+    // the finest level of an apply from an FP32 vector reads b = r32 itself (never copied, see apply)
+    const bool nat = finest && in32_;
+    if (csplit && rr_fits(nc)) {
+        const RrShape sh = rr_shape(nc, ctx_.sm_count);
+        const bool fx = first_fused32(l + 1);
+        auto pick = [&](auto nn) {
+            constexpr int NN = decltype(nn)::value;
+            return nat ? (fx ? k_residual_restrict<NN, true, true> : k_residual_restrict<NN, true, false>)
+                       : (fx ? k_residual_restrict<NN, false, true> : k_residual_restrict<NN, false, false>);
+        };
+        auto k = n == 255 ? pick(std::integral_constant<int, 255>{})
+               : n == 127 ? pick(std::integral_constant<int, 127>{})
+               : n == 63  ? pick(std::integral_constant<int, 63>{})
+                          : pick(std::integral_constant<int, 0>{});
+        launch_pdl(k, sh.grid, sh.block, 0, s, x, nat ? in32_ : b, C.b32.p, C.bs32.p, C.xs, g, nc, gc.half,
+                   (float)L.h2inv, (float)C.inv, sh.depth);
+        ctx_.count_launch();
+    } else {
         // two planes a thread sharing their i-neighbours (a four-plane march without the sharing took 80
         // registers)
         const dim3 rgd(((n + 1) / 2 + BX - 1) / BX, (n + BY - 1) / BY, (n + 1) / 2);
-        // the finest level of an apply from an FP32 vector reads b = r32 itself (never copied, see apply)
-        if (finest && in32_) launch_pdl(k_residual_split<true>, rgd, blk, 0, s, x, in32_, r, g, (float)L.h2inv);
+        if (nat) launch_pdl(k_residual_split<true>, rgd, blk, 0, s, x, in32_, r, g, (float)L.h2inv);
         else launch_pdl(k_residual_split<false>, rgd, blk, 0, s, x, b, r, g, (float)L.h2inv);
-        ctx_.count_launch();
+        const dim3 rg((nc + BX - 1) / BX, (nc + BY - 1) / BY, nc);
+        const dim3 rg2((nc + BX - 1) / BX, (nc + BY - 1) / BY, (nc + 1) / 2);  // two coarse planes a thread
+        if (csplit && first_fused32(l + 1))
+            launch_pdl(k_restrict_split<true>, rg2, blk, 0, s, r, C.b32.p, C.bs32.p, C.xs, n, nc, gc.half, (float)C.inv);
+        else if (csplit)
+            launch_pdl(k_restrict_split<false>, rg2, blk, 0, s, r, C.b32.p, C.bs32.p, C.xs, n, nc, gc.half, (float)C.inv);
+        else
+            launch_pdl(k_restrict<float>, rg, blk, 0, s, (const float*)r, C.b32.p, C.bs32.p, n, nc, C.inv, (float*)nullptr);
+        ctx_.count_launch(2);
     }
-    const Split gc = make_split(nc);
-    const dim3 rg((nc + BX - 1) / BX, (nc + BY - 1) / BY, nc);
-    const dim3 rg2((nc + BX - 1) / BX, (nc + BY - 1) / BY, (nc + 1) / 2);  // two coarse planes a thread
-    if (csplit && first_fused32(l + 1))
-        launch_pdl(k_restrict_split<true>, rg2, blk, 0, s, r, C.b32.p, C.bs32.p, C.xs, n, nc, gc.half, (float)C.inv);
-    else if (csplit)
-        launch_pdl(k_restrict_split<false>, rg2, blk, 0, s, r, C.b32.p, C.bs32.p, C.xs, n, nc, gc.half, (float)C.inv);
-    else
-        launch_pdl(k_restrict<float>, rg, blk, 0, s, (const float*)r, C.b32.p, C.bs32.p, n, nc, C.inv, (float*)nullptr);
-    ctx_.count_launch();
     if (l == 0) coarse_cycle();
     else cycle32(l + 1);
     const dim3 cg((nc + 1 + BX - 1) / BX, (nc + 1 + BY - 1) / BY, nc + 1);
