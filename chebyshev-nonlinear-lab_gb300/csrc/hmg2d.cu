@@ -12,12 +12,12 @@
 //
 // A cycle is many short steps (11 a level), so what bounds it is launches: one host launch a step and field
 // took 17.4 ms of a Burgers solve at 255^2 whose kernels ran 9 ms.  Hence: u and v go through one cycle
-// together (blockIdx.z = field); programmatic dependent launch; the levels below the finest in one CUDA
-// graph; and the levels of n <= 31 in one CTA a field, in shared memory (k_hmg_tail), where a step
-// is a block barrier.  At 31^2 a pass is 2,200 cycles of one SM's FP64 pipe, about what a launch costs;
-// at 63^2 it would be four times that, so that level stays launched.  The Burgers solve at 255^2 went from 17.5
-// to 4.3 ms; a cycle of both fields is ~110 us there, 37 of them the tail (44 steps, each bound by the
-// latency of its nine dependent FP64 operations or, at 31^2, by the FP64 pipe).
+// together (blockIdx.z = field); programmatic dependent launch; the levels below the finest in one CUDA graph; the
+// levels of 15 < n <= 127 in two tiled kernels each, on as many SMs as there are, where a step is a block barrier; and
+// the levels below in one CTA a field, in shared memory (k_hmg_tail).  The Burgers solve at 255^2 went from 17.5 to
+// 3.25 ms; a cycle of both fields is 82 us there (110 with 63^2 and 127^2 launched pass by pass and 31^2 in the tail):
+// 30 of them the finest level's 11 launches, 16 the tail (steps bound by the latency of their nine dependent FP64
+// operations), 11 each the levels between.
 #include <cmath>
 #include <limits>
 
@@ -30,6 +30,8 @@ struct HelmholtzMG2D::Level {
     int n = 0;
     double s = 0.0;  // nu / h^2 of this level
     DeviceArray<double> x, b;
+    int T = 0;              // > 0: run by the tiled kernels, T x T coarse points a block
+    DeviceArray<double> y;  // tiled: x on its way down
 };
 
 namespace {
@@ -140,10 +142,11 @@ __global__ void __launch_bounds__(BX* BY) k_hprolong(const double* __restrict__ 
 }
 
 // ------------------------------------------------------------------------------------------
-// The levels of n <= kTailTop in one CTA a field: x of each level with a halo of zeros, pitch m = (n + 2) | 1, the
+// The levels of n <= kTileTail (kTailTop where no tiled level applies) in one CTA a field: x of each level with a halo of zeros, pitch m = (n + 2) | 1, the
 // two parities of the padded index (the colours) stored apart, so that a pass reads one half and writes the other;
 // b and the residual in natural order.  The arithmetic is the launched kernels' operation for operation.
 constexpr int kTailTop = 31, kTailMax = 6, kTailThreads = 512;  // 31, 15, 7, 3, 1
+constexpr int kTileTop = 127, kTileTail = 15;                   // the levels of the tiled kernels, below
 struct HTailLvl {
     HLvl L;
     int m, H, offX, offB;  // pitch, elements of one parity of x, element offsets in shared memory
@@ -154,6 +157,153 @@ struct HTail {
 };
 
 extern __shared__ __align__(16) double htail_smem[];
+
+// ------------------------------------------------------------------------------------------
+// Levels of kTileTail < n <= kTileTop in two kernels, one on the way down (pre-smoothing from x = 0, residual,
+// restriction) and one on the way up (prolongation, post-smoothing).  A block owns T x T coarse points and the fine
+// points 2I, 2I + 1 of them (its last row and column also 2I + 2), and runs every pass on a region that shrinks by a
+// point on each side a pass, so that no block needs another's values within the kernel: the points around its own are
+// computed again.  Thread (i, jj) of the region, in linear order, holds b of the pair of points 2jj, 2jj + 1 of row i;
+// x is in shared memory with zeros around it and outside the grid.  The arithmetic is the launched kernels' operation
+// for operation.  x goes down in one array and comes up in another, as neighbours read it.
+// Bound by the latency of a pass's nine dependent FP64 operations (63^2 and below) or the FP64 pipe.  A cycle of two
+// fields: 31^2 37 -> 28.4 us, 63^2 and 127^2 11 to 12 us a level (11 launches: 24).
+struct HTile {
+    HLvl L;
+    int nc, T, S, np, sweeps;  // S x S fine points of the region, np = (S + 1) / 2 pairs a row
+};
+
+__device__ __forceinline__ void htile_pass(double* X, int P, double b, const HLvl& L, bool first) {
+    double nb = 0.0;
+    if (!first) {
+        const int m = P;
+        nb = nb + X[-m];
+        nb = nb + X[m];
+        nb = nb + X[-1];
+        nb = nb + X[1];
+    }
+    *X = div_by_recip(b + L.s * nb, L.den, L.rden);
+}
+
+__global__ void __launch_bounds__(1024) k_htile_down(const double* __restrict__ b, double* __restrict__ x,
+                                                     double* __restrict__ bc, const __grid_constant__ HTile t) {
+    const int n = t.L.n, nc = t.nc, S = t.S, m = S + 2, h = 2 * t.sweeps;
+    double* X = htail_smem;           // (S + 2)^2
+    double* R = htail_smem + m * m;   // (2T + 1)^2
+    const int nt = blockDim.x, tid = threadIdx.x;
+    for (int q = tid; q < m * m; q += nt) X[q] = 0.0;
+    const int C0i = blockIdx.y * t.T, C0j = blockIdx.x * t.T;
+    const int ri = tid / t.np, rj = 2 * (tid - ri * t.np);      // region row, first column of the pair
+    const int i = 2 * C0i - h + ri, j0 = 2 * C0j - h + rj;      // grid row, column
+    const bool row = ri < S && i >= 0 && i < n;
+    bool in[2];
+    double bv[2], xv[2];
+    pdl_wait();
+    pdl_trigger();
+    const size_t f0 = (size_t)blockIdx.z * n * n;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        in[q] = row && rj + q < S && j0 + q >= 0 && j0 + q < n;
+        bv[q] = in[q] ? b[f0 + (size_t)i * n + j0 + q] : 0.0;
+        xv[q] = 0.0;
+    }
+    double* Xp = X + (ri + 1) * m + rj + 1;
+    __syncthreads();
+#pragma unroll 1
+    for (int p = 0; p < h; ++p) {  // colours 0, 1, 0, 1, ...; the region of pass p starts p points further in
+        const int q = (i + j0 + p) & 1;  // the member of the pair of this colour
+        const int c = rj + q;
+        if ((q ? in[1] : in[0]) && ri >= p && ri < S - p && c >= p && c < S - p)
+            htile_pass(Xp + q, m, q ? bv[1] : bv[0], t.L, p == 0);
+        __syncthreads();
+    }
+    // the residual of rows and columns 2 C0 .. 2 C0 + 2T
+    const int rn = 2 * t.T + 1;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int a = ri - h, c = rj + q - h;
+        if (!in[q] || a < 0 || a >= rn || c < 0 || c >= rn) continue;
+        const double* P = Xp + q;
+        const double xc = *P;
+        double nb = 0.0;
+        nb = nb + P[-m];
+        nb = nb + P[m];
+        nb = nb + P[-1];
+        nb = nb + P[1];
+        R[a * rn + c] = bv[q] - (t.L.alpha * xc + t.L.s * (4.0 * xc - nb));
+        const bool oi = a < rn - 1 || C0i + t.T >= nc, oj = c < rn - 1 || C0j + t.T >= nc;
+        if (oi && oj) x[f0 + (size_t)i * n + j0 + q] = xc;
+    }
+    __syncthreads();
+    const int I = tid / t.T, J = tid - I * t.T;
+    if (I < t.T && C0i + I < nc && C0j + J < nc) {
+        const double w[3] = {0.25, 0.5, 0.25};
+        const double* r = R + 2 * I * rn + 2 * J;
+        double acc = 0.0;
+#pragma unroll
+        for (int a = 0; a < 9; ++a) acc = __fma_rn(w[a / 3] * w[a % 3], r[(a / 3) * rn + a % 3], acc);
+        bc[((size_t)blockIdx.z * nc + C0i + I) * nc + C0j + J] = acc;
+    }
+}
+
+__global__ void __launch_bounds__(1024) k_htile_up(const double* __restrict__ b, const double* __restrict__ xd,
+                                                   const double* __restrict__ xc, double* __restrict__ x,
+                                                   const __grid_constant__ HTile t) {
+    const int n = t.L.n, nc = t.nc, S = t.S, m = S + 2, h = 2 * t.sweeps;
+    double* X = htail_smem;
+    const int nt = blockDim.x, tid = threadIdx.x;
+    for (int q = tid; q < m * m; q += nt) X[q] = 0.0;
+    const int C0i = blockIdx.y * t.T, C0j = blockIdx.x * t.T;
+    const int ri = tid / t.np, rj = 2 * (tid - ri * t.np);
+    const int i = 2 * C0i - h + ri, j0 = 2 * C0j - h + rj;
+    const bool row = ri < S && i >= 0 && i < n;
+    bool in[2];
+    double bv[2];
+    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    const size_t f0 = (size_t)blockIdx.z * n * n;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        in[q] = row && rj + q < S && j0 + q >= 0 && j0 + q < n;
+        bv[q] = in[q] ? b[f0 + (size_t)i * n + j0 + q] : 0.0;
+    }
+    double* Xp = X + (ri + 1) * m + rj + 1;
+    {  // the colour-0 point of the pair, corrected as k_hprolong does
+        const int q = (i + j0) & 1, j = j0 + q;
+        if (q ? in[1] : in[0]) {
+            const int I0 = ((i + 1) >> 1) - 1, J0 = ((j + 1) >> 1) - 1;
+            const double w = (i & 1 ? 1.0 : 0.5) * (j & 1 ? 1.0 : 0.5);
+            double v[4];
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const int I = I0 + (g >> 1), J = J0 + (g & 1);
+                const bool has = !((g >> 1) && (i & 1)) && !((g & 1) && (j & 1)) && I >= 0 && I < nc && J >= 0 && J < nc;
+                v[g] = has ? xc[((size_t)blockIdx.z * nc + I) * nc + J] : 0.0;
+            }
+            const double xo = xd[f0 + (size_t)i * n + j];
+            double acc = 0.0;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) acc = __fma_rn(w, v[g], acc);
+            Xp[q] = xo + acc;
+        }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int p = 0; p < h; ++p) {  // colours 1, 0, 1, 0, ...
+        const int q = (i + j0 + p + 1) & 1, c = rj + q, d = p + 1;
+        if ((q ? in[1] : in[0]) && ri >= d && ri < S - d && c >= d && c < S - d)
+            htile_pass(Xp + q, m, q ? bv[1] : bv[0], t.L, false);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int a = ri - h, c = rj + q - h, rn = 2 * t.T + 1;
+        if (!in[q] || a < 0 || a >= rn || c < 0 || c >= rn) continue;
+        const bool oi = a < rn - 1 || C0i + t.T >= nc, oj = c < rn - 1 || C0j + t.T >= nc;
+        if (oi && oj) x[f0 + (size_t)i * n + j0 + q] = Xp[q];
+    }
+}
 
 // x at padded index P
 __device__ __forceinline__ double& hx(double* X, int H, int P) { return X[(P & 1) * H + (P >> 1)]; }
@@ -275,6 +425,21 @@ __global__ void __launch_bounds__(kTailThreads) k_hmg_tail(const double* b, doub
 
 }  // namespace
 
+// The coarse points T a side of a tile block, 0 for a level that the tiled kernels do not take: the smallest T whose
+// blocks all have an SM to themselves, for 1 to 3 sweeps and kTileTail < n <= kTileTop.  Above, the points computed
+// again cost the FP64 pipe more than the launches did (255^2, 1.6 times the points: the cycle 90 us against 82); below,
+// one CTA's tail is faster (15^2: 19.5 us against 21.0).
+static int tile_size(int n, int fields, int pre, int post, int sm_count) {
+    if (n > kTileTop || n <= kTileTail || pre < 1 || pre > 3 || post < 1 || post > 3) return 0;
+    const int nc = (n - 1) / 2;
+    int T = 1;
+    while ((long long)((nc + T - 1) / T) * ((nc + T - 1) / T) * fields > sm_count) {
+        if (++T > nc) return 0;
+    }
+    const int S = 2 * T + 1 + 4 * std::max(pre, post);
+    return S * ((S + 1) / 2) <= 1024 ? T : 0;
+}
+
 static HLvl hlvl(int n, double s, double alpha) {
     const double den = alpha + 4.0 * s;
     // recip_for_div on the host: RN(1/den) inside the exponent range the correction needs, else 0
@@ -298,17 +463,23 @@ HelmholtzMG2D::HelmholtzMG2D(Context& ctx, size_t n, double alpha, double nu, in
         m = (m - 1) / 2;
         s /= 4.0;
     }
-    for (size_t l = 0; l < levels_.size(); ++l)
-        if (levels_[l]->n <= kTailTop) {  // (at most 31, 15, 7, 3, 1 follow)
+    for (size_t l = 0; l < levels_.size(); ++l) {
+        Level& L = *levels_[l];
+        const bool coarser = l + 1 < levels_.size();
+        L.T = coarser ? tile_size(L.n, fields, pre, post, ctx.sm_count) : 0;
+        if (L.n <= (L.T ? kTileTail : kTailTop)) {  // (at most 31, 15, 7, 3, 1 follow)
+            L.T = 0;
             tail_l_ = l;
             break;
         }
+        if (L.T) L.y.resize((size_t)fields * L.n * L.n);
+    }
     for (size_t l = 1; l < levels_.size() && l <= tail_l_; ++l) {
         const size_t Nl = (size_t)fields * levels_[l]->n * levels_[l]->n;
         levels_[l]->x.resize(Nl);
         levels_[l]->b.resize(Nl);
     }
-    if (tail_l_ > 0) resid_.resize(fields * N0_);
+    if (tail_l_ > 0 && !levels_[0]->T) resid_.resize(fields * N0_);
     set_dynamic_smem_limit(ctx_, k_hmg_tail);
 }
 
@@ -381,6 +552,26 @@ void HelmholtzMG2D::cycle(size_t l) {
     }
     const HLvl K = hlvl(n, L.s, alpha_);
     cudaStream_t st = ctx_.stream;
+    if (L.T) {
+        Level& C = *levels_[l + 1];
+        auto tile = [&](int sweeps) {
+            const int S = 2 * L.T + 1 + 4 * sweeps;
+            return HTile{K, C.n, L.T, S, (S + 1) / 2, sweeps};
+        };
+        const unsigned k = (unsigned)((C.n + L.T - 1) / L.T);
+        const dim3 grid(k, k, (unsigned)fields_);
+        auto threads = [](const HTile& t) { return dim3((unsigned)((t.S * t.np + 31) / 32 * 32)); };
+        auto smem = [](const HTile& t) { return ((size_t)(t.S + 2) * (t.S + 2) + (2 * t.T + 1) * (2 * t.T + 1)) * sizeof(double); };
+        const HTile down = tile(pre_), up = tile(post_);
+        launch_pdl(k_htile_down, grid, threads(down), smem(down), st, b, L.y.p, C.b.p, down);
+        ctx_.count_launch();
+        if (l == 0) coarse_cycle();
+        else cycle(l + 1);
+        launch_pdl(k_htile_up, grid, threads(up), smem(up), st, b, (const double*)L.y.p, (const double*)C.x.p, x, up);
+        ctx_.count_launch();
+        ctx_.check_launch("hmg2d tiled level");
+        return;
+    }
     const dim3 blk(BX, BY);
     const unsigned nf = (unsigned)fields_;
     const dim3 cg(((n + 1) / 2 + BX - 1) / BX, (n + BY - 1) / BY, nf);
