@@ -746,6 +746,162 @@ __global__ void __launch_bounds__(256) k_bmg_prolong_pass(const T* __restrict__ 
     st2(X, p10, u, v);
 }
 
+// The middle levels of the FP32 cycle (kBTileTail < n <= kBTileTop below the finest, a coarser one below) in two
+// kernels each, one on the way down (pre-smoothing from x = 0, residual, restriction) and one on the way up
+// (prolongation, post-smoothing).  A block owns T x T coarse points and the fine points (2I + {0, 1}, 2J + {0, 1}) of
+// them, and runs every pass on a region that shrinks by a point on each side a pass: it computes the points around its
+// own again instead of waiting for other blocks.  Thread (i, jj) of the region, in linear order, holds b and K of a
+// pair of neighbouring points; x is in shared memory.  x goes down in one array and comes up in another, as the blocks
+// around read it.  The arithmetic is the launched kernels' operation for operation.
+// Bound by the latency of a pass and its barrier: 4.2 + 3.0 us on 256^2, 2.4 + 2.1 on 32^2, for eight launches a level
+// (256^2 15 us) or 20 us of the one-CTA tail (64^2).  512^2 needs two waves of blocks and stays launched.
+constexpr int kBTileTop = 256, kBTileTail = 16;
+struct BTile {
+    LvlArgs<float> L;
+    int T, S, np, sweeps;  // S x S points of the region, np = (S + 1) / 2 pairs a row
+};
+inline BTile btile(const LvlArgs<float>& L, int T, int sweeps, bool down) {
+    const int S = 2 * T + 4 * sweeps + (down ? 1 : 0);
+    return BTile{L, T, S, (S + 1) / 2, sweeps};
+}
+inline int btile_threads(const BTile& t) { return (t.S * t.np + 31) / 32 * 32; }
+inline size_t btile_smem(const BTile& t) {
+    return ((size_t)t.S * t.S + (size_t)(2 * t.T + 1) * (2 * t.T + 1)) * sizeof(float2);
+}
+// T of a level, 0 where the tiled kernels do not take it: the smallest whose blocks all have an SM to themselves.
+inline int btile_size(int n, int pre, int post, int sm_count) {
+    if (n <= kBTileTail || n > kBTileTop || pre > 3 || post > 3) return 0;
+    const int nc = n / 2;
+    int T = 1;
+    while (((nc + T - 1) / T) * ((nc + T - 1) / T) > sm_count) ++T;
+    const LvlArgs<float> L{};
+    return std::max(btile_threads(btile(L, T, pre, true)), btile_threads(btile(L, T, post, false))) <= 1024 ? T : 0;
+}
+
+__device__ __forceinline__ int wrap(int i, int n) {
+    i %= n;
+    return i < 0 ? i + n : i;
+}
+
+// ((W + E) + S) + N around a point of the region
+__device__ __forceinline__ float2 btile_sum(const float2* X, int S) {
+    const float2 w = X[-1], e = X[1], s = X[-S], n = X[S];
+    return make_float2(((w.x + e.x) + s.x) + n.x, ((w.y + e.y) + s.y) + n.y);
+}
+
+extern __shared__ __align__(16) float2 btile_smem_x[];
+
+__global__ void __launch_bounds__(1024) k_btile_down(const float* __restrict__ Bv, const float* __restrict__ K,
+                                                     float* __restrict__ Y, float* __restrict__ Bc,
+                                                     const __grid_constant__ BTile t) {
+    float2* X = btile_smem_x;        // S^2
+    float2* R = X + t.S * t.S;       // (2T + 1)^2: rows and columns 2 C0 - 1 .. 2 C0 + 2T - 1
+    const int n = t.L.n, nc = n / 2, S = t.S, h = 2 * t.sweeps, rn = 2 * t.T + 1;
+    const int C0i = blockIdx.y * t.T, C0j = blockIdx.x * t.T;
+    const int ri = (int)threadIdx.x / t.np, rj = 2 * ((int)threadIdx.x - ri * t.np);
+    const int i = 2 * C0i - h - 1 + ri, j0 = 2 * C0j - h - 1 + rj;
+    const int iw = wrap(i, n);
+    float2 b[2];
+    Blk<float> k[2];
+    bool in[2];
+    pdl_wait();
+    pdl_trigger();
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        in[q] = ri < S && rj + q < S;
+        if (!in[q]) continue;
+        const size_t p = pidx(n, iw, wrap(j0 + q, n));
+        b[q] = ld2(Bv, p);
+        k[q] = load_blk(K, p);
+    }
+    float2* Xp = X + ri * S + rj;
+#pragma unroll 1
+    for (int p = 0; p < h; ++p) {  // colours 0, 1, 0, 1, ...
+        const int q = (i + j0 + p) & 1, c = rj + q;
+        if (ri >= p && ri < S - p && c >= p && c < S - p) {
+            const float2 s = p == 0 ? make_float2(0.0f, 0.0f) : btile_sum(Xp + q, S);
+            float u, v;
+            block_update(q ? k[1] : k[0], t.L.su, t.L.sv, t.L.su4, t.L.sv4, q ? b[1].x : b[0].x, q ? b[1].y : b[0].y, s.x,
+                         s.y, u, v);
+            Xp[q] = make_float2(u, v);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int a = ri - h, c = rj + q - h;
+        if (!in[q] || a < 0 || a >= rn || c < 0 || c >= rn) continue;
+        const float2 x = Xp[q], s = btile_sum(Xp + q, S);
+        float2 r;
+        resid_value(k[q], x, b[q], s.x, s.y, t.L.su, t.L.sv, r.x, r.y);
+        R[a * rn + c] = r;
+        if (a > 0 && c > 0 && i < n && j0 + q < n) st2(Y, pidx(n, i, j0 + q), x.x, x.y);
+    }
+    __syncthreads();
+    const int I = (int)threadIdx.x / t.T, J = (int)threadIdx.x - I * t.T;
+    if (I < t.T && C0i + I < nc && C0j + J < nc) {
+        const float2* f = R + (2 * I + 1) * rn + 2 * J + 1;
+        const float u = fw9(f[0].x, f[-1].x, f[1].x, f[-rn].x, f[rn].x, f[-rn - 1].x, f[-rn + 1].x, f[rn - 1].x,
+                            f[rn + 1].x);
+        const float v = fw9(f[0].y, f[-1].y, f[1].y, f[-rn].y, f[rn].y, f[-rn - 1].y, f[-rn + 1].y, f[rn - 1].y,
+                            f[rn + 1].y);
+        st2(Bc, pidx(nc, C0i + I, C0j + J), u, v);
+    }
+}
+
+__global__ void __launch_bounds__(1024) k_btile_up(const float* __restrict__ Bv, const float* __restrict__ K,
+                                                   const float* __restrict__ Y, const float* __restrict__ Xc,
+                                                   float* __restrict__ Xo, const __grid_constant__ BTile t) {
+    float2* X = btile_smem_x;
+    const int n = t.L.n, nc = n / 2, S = t.S, h = 2 * t.sweeps;
+    const int ri = (int)threadIdx.x / t.np, rj = 2 * ((int)threadIdx.x - ri * t.np);
+    const int i = 2 * (int)blockIdx.y * t.T - h + ri, j0 = 2 * (int)blockIdx.x * t.T - h + rj;
+    const int iw = wrap(i, n);
+    const bool row = ri < S;  // (S is even: both points of a pair are in the region)
+    float2 b[2];
+    Blk<float> k[2];
+    pdl_wait();
+    pdl_trigger();
+    float2* Xp = X + ri * S + rj;
+    if (row) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const size_t p = pidx(n, iw, wrap(j0 + q, n));
+            b[q] = ld2(Bv, p);
+            k[q] = load_blk(K, p);
+        }
+        // the pair's colour-0 point, corrected: (even, even) or (odd, odd)
+        const int q = (i + j0) & 1, jw = wrap(j0 + q, n);
+        const int I = iw >> 1, J = jw >> 1;
+        const float2 x = ld2(Y, pidx(n, iw, jw)), c00 = ld2(Xc, pidx(nc, I, J));
+        float2 d = c00;
+        if (iw & 1) {
+            const int I1 = I + 1 == nc ? 0 : I + 1, J1 = J + 1 == nc ? 0 : J + 1;
+            d = interp11(c00, ld2(Xc, pidx(nc, I1, J)), ld2(Xc, pidx(nc, I, J1)), ld2(Xc, pidx(nc, I1, J1)));
+        }
+        Xp[q] = add2(x, d);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int p = 0; p < h; ++p) {  // colours 1, 0, 1, 0, ...
+        const int q = (i + j0 + p + 1) & 1, c = rj + q, e = p + 1;
+        if (ri >= e && ri < S - e && c >= e && c < S - e) {
+            const float2 s = btile_sum(Xp + q, S);
+            float u, v;
+            block_update(q ? k[1] : k[0], t.L.su, t.L.sv, t.L.su4, t.L.sv4, q ? b[1].x : b[0].x, q ? b[1].y : b[0].y, s.x,
+                         s.y, u, v);
+            Xp[q] = make_float2(u, v);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int a = ri - h, c = rj + q - h;
+        if (a < 0 || a >= 2 * t.T || c < 0 || c >= 2 * t.T || i >= n || j0 + q >= n) continue;
+        st2(Xo, pidx(n, i, j0 + q), Xp[q].x, Xp[q].y);
+    }
+}
+
 // The coarsest level in one block: x = 0, then `sweeps` red-black sweeps (colour 0, 1).
 template <class T>
 __global__ void __launch_bounds__(1024) k_bmg_coarsest(T* __restrict__ X, const T* __restrict__ Bv,
@@ -1228,6 +1384,8 @@ struct BrussMG2D::Level {
     int n;
     double su, sv;
     DeviceArray<double> x, b, k;  // level pairs and blocks in the multigrid's precision
+    int T = 0;                    // > 0: run by the tiled kernels, T x T coarse points a block
+    DeviceArray<double> y;        // tiled: x on its way down
 };
 
 BrussMG2D::BrussMG2D(Context& ctx, size_t n, const numa_brusselator2d_params& p, int precision, int pre, int post)
@@ -1257,11 +1415,16 @@ BrussMG2D::BrussMG2D(Context& ctx, size_t n, const numa_brusselator2d_params& p,
     // levels below the finest with n <= 64 (FP32) or n <= 32 (FP64) run as one block: x, b and K,
     // 8 (64^2 + 32^2 + ...) values, at most 175 KB of shared memory
     const int tail_max_n = precision == NUMA_GPU_FP64 ? kBmgTailMaxN / 2 : kBmgTailMaxN;
-    for (size_t l = 1; l < levels_.size(); ++l)
-        if (levels_[l]->n <= tail_max_n) {
+    for (size_t l = 1; l < levels_.size(); ++l) {
+        Level& L = *levels_[l];
+        if (precision == NUMA_GPU_FP32 && l + 1 < levels_.size()) L.T = btile_size(L.n, pre, post, ctx.sm_count);
+        if (L.T) {
+            L.y.resize(L.x.n);
+        } else if (L.n <= tail_max_n) {
             tail_first_ = (int)l;
             break;
         }
+    }
     if (tail_first_ > 0) {
         std::vector<TailLvl> d;
         size_t off = 0;
@@ -1321,7 +1484,7 @@ void BrussMG2D::set_state(const double* w) {
 // Whether level l's first smoothing pass is done by the restriction that forms its right-hand side.
 template <class T>
 bool BrussMG2D::first_fused(size_t l) const {
-    return sizeof(T) == 4 && l > 0 && (int)l != tail_first_ && l + 1 < levels_.size();
+    return sizeof(T) == 4 && l > 0 && (int)l != tail_first_ && !levels_[l]->T && l + 1 < levels_.size();
 }
 
 template <class T>
@@ -1343,6 +1506,21 @@ void BrussMG2D::cycle(size_t l) {
                                                   post_, kBmgCoarsestSweeps, Bv, X);
         ctx_.count_launch();
         return;
+    }
+    if constexpr (sizeof(T) == 4) {
+        if (L.T) {
+            Level& C = *levels_[l + 1];
+            const unsigned g = (unsigned)((C.n + L.T - 1) / L.T);
+            const BTile down = btile(A, L.T, pre_, true), up = btile(A, L.T, post_, false);
+            launch_pdl(k_btile_down, dim3(g, g), btile_threads(down), btile_smem(down), s, (const T*)Bv, K, tp<T>(L.y),
+                       tp<T>(C.b), down);
+            ctx_.count_launch();
+            cycle<T>(l + 1);
+            launch_pdl(k_btile_up, dim3(g, g), btile_threads(up), btile_smem(up), s, (const T*)Bv, K,
+                       (const T*)tp<T>(L.y), (const T*)tp<T>(C.x), X, up);
+            ctx_.count_launch();
+            return;
+        }
     }
     if (coarsest) {
         if (finest) {

@@ -34,12 +34,12 @@ def test_residual_and_norm_over_row_chunks(gpu, oracle, n):
     assert abs(r["res0"] - np.sqrt(np.sum(f * f))) <= 1e-12 * r["res0"]
 
 
-@pytest.mark.parametrize("n", [8, 20, 24, 72, 136, 200, 264, 1000])
-@pytest.mark.parametrize("pre,post", [(2, 2), (1, 3)])
+@pytest.mark.parametrize("n", [8, 20, 24, 40, 72, 136, 200, 264, 512, 1000])
+@pytest.mark.parametrize("pre,post", [(2, 2), (1, 3), (3, 1), (4, 1)])
 def test_vcycle_tiles(gpu, oracle, n, pre, post):
     """Levels whose coarse rows end in remainders (31 coarse columns a warp) or are narrower than one,
     hierarchies ending in a large coarsest level, other sweep counts: FP64 bit for bit; FP32 within 2e-5, the
-    bound of the FP32 V-cycle's other tests."""
+    bound of the FP32 V-cycle's other tests.  FP32 levels of 16 < n <= 256 run in tiles (up to three sweeps)."""
     import numa_gpu as G
 
     N = 2 * n * n
