@@ -942,16 +942,74 @@ struct TailLvl {
     LvlArgs<double> d;  // the level's constants in FP64 and in FP32 (formed on the host: one SM's
     LvlArgs<float> f;   // FP64 pipe would take tens of microseconds to convert them per pass)
 };
+constexpr int kBmgTailLevels = 6;  // at most 64, 32, 16, 8, 4
 template <class T> __device__ __forceinline__ const LvlArgs<T>& tail_args(const TailLvl& L);
 template <> __device__ __forceinline__ const LvlArgs<double>& tail_args<double>(const TailLvl& L) { return L.d; }
 template <> __device__ __forceinline__ const LvlArgs<float>& tail_args<float>(const TailLvl& L) { return L.f; }
+
+// The coarsest level of a tail by one warp (n even, n <= 8): x = 0, then `sweeps` red-black sweeps.  A lane holds one
+// point of each colour, with its b, K and determinant, and takes its neighbours' values from their lanes; a pass is
+// the latency of eight shuffles and a block update.  (With the values in shared memory and the addresses formed again
+// each pass, 60 passes on 4 x 4 points made the tail of 16^2 24.5 us; so 15.7.)
+template <class T>
+__device__ __forceinline__ void tail_coarsest_warp(T* X, int n, const LvlArgs<T>& A, int sweeps) {
+    const int half = n / 2, cnt = n * half;
+    const int lane = threadIdx.x, idx = lane < cnt ? lane : 0;
+    const int i = idx / half, jj = idx - i * half;
+    const int im = i == 0 ? n - 1 : i - 1, ip = i + 1 == n ? 0 : i + 1;
+    const int ls = im * half + jj, ln = ip * half + jj;
+    const T* Bv = X + 2 * n * n;
+    const T* K = X + 4 * n * n;
+    T bu[2], bv[2], m11[2], m22[2], k12[2], k21[2], det[2], xu[2], xv[2];
+    int lw[2], le[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const auto b = ld2(Bv, c * cnt + idx);
+        const Blk<T> k = load_blk_s(K, c * cnt + idx);
+        bu[c] = b.x;
+        bv[c] = b.y;
+        m11[c] = k.k11 + A.su4;
+        m22[c] = k.k22 + A.sv4;
+        k12[c] = k.k12;
+        k21[c] = k.k21;
+        det[c] = m11[c] * m22[c] - k12[c] * k21[c];
+        xu[c] = xv[c] = T(0);
+        const bool right = (i + c) & 1;  // the point's j is 2jj + 1
+        lw[c] = i * half + (right ? jj : jj == 0 ? half - 1 : jj - 1);
+        le[c] = i * half + (!right ? jj : jj + 1 == half ? 0 : jj + 1);
+    }
+    constexpr unsigned all = 0xffffffffu;
+#pragma unroll 1
+    for (int s = 0; s < sweeps; ++s) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const T ou = xu[c ^ 1], ov = xv[c ^ 1];
+            const T Su = ((__shfl_sync(all, ou, lw[c]) + __shfl_sync(all, ou, le[c])) + __shfl_sync(all, ou, ls)) +
+                         __shfl_sync(all, ou, ln);
+            const T Sv = ((__shfl_sync(all, ov, lw[c]) + __shfl_sync(all, ov, le[c])) + __shfl_sync(all, ov, ls)) +
+                         __shfl_sync(all, ov, ln);
+            const T ru = bu[c] + A.su * Su, rv = bv[c] + A.sv * Sv;  // block_update's steps
+            xu[c] = (m22[c] * ru - k12[c] * rv) / det[c];
+            xv[c] = (m11[c] * rv - k21[c] * ru) / det[c];
+        }
+    }
+    if (lane < cnt) {
+        st2(X, idx, xu[0], xv[0]);
+        st2(X, cnt + idx, xu[1], xv[1]);
+    }
+    __syncwarp();
+}
 
 // threads of the one-CTA tail: 1024 in FP32 (64 registers, no spills), 512 in FP64 (which would spill at 1024)
 template <class T>
 constexpr int kBmgTailThreads = sizeof(T) == 4 ? 1024 : 512;
 template <class T>
-__global__ void __launch_bounds__(kBmgTailThreads<T>, 1) k_bmg_tail(const TailLvl* __restrict__ desc, int count, int pre, int post,
+__global__ void __launch_bounds__(kBmgTailThreads<T>, 1) k_bmg_tail(const TailLvl* __restrict__ descs, int count, int pre, int post,
                                                      int sweeps, const T* __restrict__ Bin, T* __restrict__ Xout) {
+    __shared__ TailLvl desc[kBmgTailLevels];  // (written once, when the hierarchy is made)
+    for (int q = threadIdx.x; q < count * (int)(sizeof(TailLvl) / 4); q += blockDim.x)
+        reinterpret_cast<int*>(desc)[q] = reinterpret_cast<const int*>(descs)[q];
+    __syncthreads();
     pdl_wait();
     pdl_trigger();
     extern __shared__ __align__(16) unsigned char bmg_smem[];
@@ -1059,6 +1117,10 @@ __global__ void __launch_bounds__(kBmgTailThreads<T>, 1) k_bmg_tail(const TailLv
         const bool small = kc >= kw;
         const int tid = threadIdx.x, nt = small ? 32 : blockDim.x;
         T* X = base + desc[kc].off;
+        if (small) {  // n <= 8: a lane has one point of each colour
+            tail_coarsest_warp(X, n, tail_args<T>(desc[kc]), sweeps);
+            return;
+        }
         for (int q = tid; q < 2 * n * n; q += nt) X[q] = T(0);
         if (small) __syncwarp();
         else __syncthreads();
