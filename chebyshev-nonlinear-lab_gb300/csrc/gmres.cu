@@ -187,8 +187,10 @@ __global__ void __launch_bounds__(kRedThreads) k_icwy_dots(const double* __restr
     }
 }
 
-// w -= sum_{r <= j} h_r V_r, one FMA a term in r order, and *norm = ||w||.  Two elements a thread at a time: the
-// terms of one are a chain.
+// w -= sum_{r <= j} h_r V_r, one FMA a term in r order, and *norm = ||w||.  Bound on short vectors by the FP64 pipe of
+// the SMs that have a block (8 warps fill it: 32 terms are 4,096 cycles) and the latency of the loads, eight terms
+// ahead.  Over the columns 5 to 32 of a cycle at 31^3 9.4 us a
+// kernel, 11.7 with two elements a thread at a time, which left 59 SMs with a block.
 __global__ void __launch_bounds__(kRedThreads) k_icwy_update(double* __restrict__ w, const double* __restrict__ V,
                                                              size_t N, int j, const double* __restrict__ hcol,
                                                              RedArgs red, StoreNormAt fin, HostOut host) {
@@ -196,26 +198,24 @@ __global__ void __launch_bounds__(kRedThreads) k_icwy_update(double* __restrict_
     pdl_trigger();
     __shared__ double h[kIcwyMax];
     __shared__ double sm[1][32];
-    if (threadIdx.x <= j) h[threadIdx.x] = hcol[threadIdx.x];
+    if (threadIdx.x < kIcwyMax) h[threadIdx.x] = threadIdx.x <= j ? hcol[threadIdx.x] : 0.0;
     __syncthreads();
     double s[1] = {0.0};
     const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += 2 * stride) {
-        const size_t i2 = i + stride;
-        const bool two = i2 < N;
-        double wa = w[i], wb = two ? w[i2] : 0.0;
-        const double *va = V + i, *vb = V + (two ? i2 : i);
-#pragma unroll 4
-        for (int r = 0; r <= j; ++r, va += N, vb += N) {
-            wa = __fma_rn(-h[r], *va, wa);
-            wb = __fma_rn(-h[r], *vb, wb);
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += stride) {
+        double wi = w[i];
+        const double* v = V + i;
+        int r = 0;
+        for (; r + 8 <= j + 1; r += 8, v += 8 * N) {
+            double t[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) t[q] = v[q * N];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) wi = __fma_rn(-h[r + q], t[q], wi);
         }
-        w[i] = wa;
-        s[0] = __fma_rn(wa, wa, s[0]);
-        if (two) {
-            w[i2] = wb;
-            s[0] = __fma_rn(wb, wb, s[0]);
-        }
+        for (; r <= j; ++r, v += N) wi = __fma_rn(-h[r], *v, wi);
+        w[i] = wi;
+        s[0] = __fma_rn(wi, wi, s[0]);
     }
     block_sum<1>(s, sm);
     grid_reduce_finish<1>(s, red, fin, host);
@@ -752,11 +752,16 @@ void Gmres::arnoldi_mgs(size_t j, double* w) {
     const double* V = V_.p;
     if (j >= (size_t)kIcwyFrom && j < (size_t)kIcwyMax && N <= kIcwyMaxN) {
         gram_.resize(kIcwyMax * kIcwyMax);
-        const size_t blocks = (N + 2 * kRedThreads - 1) / (2 * kRedThreads);
-        // two blocks an SM for the inner products: each block's partial sums are 16 more values for the last one
-        const unsigned gd = (unsigned)std::min<size_t>(blocks, 2 * (size_t)ctx_.sm_count);
+        const size_t blocks = (N + kRedThreads - 1) / kRedThreads;
         const bool start = j == (size_t)kIcwyFrom;
-        launch_pdl(start ? k_icwy_dots<true> : k_icwy_dots<false>, dim3(gd, (unsigned)(j / 8 + 1 + start)), kRedThreads, 0,
+        const unsigned groups = (unsigned)(j / 8 + 1 + start);
+        // The inner products: one block an SM over all groups of vectors (two from 2^17 points), as few as fill the
+        // FP64 pipe, since a block's 16 sums over its warps cost what one element a thread does, and its partial sums
+        // are 16 more values for the last block (columns 5 to 32
+        // at 31^3: 12.3 us, 12.6 with a block for every 512 points and group).
+        const size_t fill = (size_t)ctx_.sm_count * (N > (size_t)1 << 17 ? 2 : 1) / groups;
+        const unsigned gd = (unsigned)std::max<size_t>(1, std::min(blocks, fill));
+        launch_pdl(start ? k_icwy_dots<true> : k_icwy_dots<false>, dim3(gd, groups), kRedThreads, 0,
                    ctx_.stream, (const double*)w, V, N, (int)j, ctx_.red, gram_.p, hcol);
         launch_pdl(k_icwy_update, (unsigned)std::min<size_t>(blocks, 8 * (size_t)ctx_.sm_count), kRedThreads, 0,
                    ctx_.stream, w, V, N, (int)j, (const double*)hcol, ctx_.red,
