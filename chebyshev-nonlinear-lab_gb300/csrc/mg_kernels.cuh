@@ -532,15 +532,16 @@ __global__ void __launch_bounds__(BX* BY) k_restrict_split(const float* __restri
 // 2.0 + 1.8 us.
 constexpr int kRrRows = 7, kRrMaxCols = 128, kRrThreads = 1024;  // threads an SM (64 registers each)
 
+// For sizes known at compile time only: with the offsets of a plane's loads formed at run time the two kernels are
+// faster (V-cycle at 191^3 222.9 us against 226.8, 223^3 322.6 against 324.0).
 template <int NN, bool BNAT, bool FIRST_X>
 __device__ __forceinline__ void residual_restrict_body(const float* __restrict__ x, const float* __restrict__ b,
                                                        float* __restrict__ bc, float* __restrict__ bsc,
-                                                       float* __restrict__ xc, const Split& g, int nc, int halfc,
+                                                       float* __restrict__ xc, const Split& g, int halfc,
                                                        float h2inv, float inv_c, int depth, int bx, int by, int bz) {
     __shared__ float2 sa[2][kRrRows + 1][kRrMaxCols];  // residuals at (2J, 2K), (2J, 2K + 1)
     __shared__ float2 sb[2][kRrRows][kRrMaxCols];      // at (2J + 1, 2K), (2J + 1, 2K + 1)
-    if (NN > 0) nc = (NN - 1) / 2;
-    const int n = NN > 0 ? NN : g.n, P = n * n;
+    constexpr int n = NN, nc = (NN - 1) / 2, P = n * n;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int Kr = bx * ((int)blockDim.x - 1) + tx, Jr = by * kRrRows + ty;
     const bool own = tx + 1 < (int)blockDim.x && Kr < nc && ty < kRrRows && Jr < nc;
@@ -646,19 +647,11 @@ __device__ __forceinline__ void residual_restrict_body(const float* __restrict__
 template <int NN, bool BNAT, bool FIRST_X>
 __global__ void __launch_bounds__(kRrMaxCols*(kRrRows + 1), kRrThreads / (kRrMaxCols * (kRrRows + 1))) k_residual_restrict(
     const float* __restrict__ x, const float* __restrict__ b, float* __restrict__ bc, float* __restrict__ bsc,
-    float* __restrict__ xc, Split g, int nc, int halfc, float h2inv, float inv_c, int depth) {
+    float* __restrict__ xc, Split g, int halfc, float h2inv, float inv_c, int depth) {
     pdl_wait();
     pdl_trigger();
-    residual_restrict_body<NN, BNAT, FIRST_X>(x, b, bc, bsc, xc, g, nc, halfc, h2inv, inv_c, depth, blockIdx.x,
-                                              blockIdx.y, blockIdx.z);
-}
-
-// Whether a level's cells fill the lanes of residual_restrict's rows (7 of 8 at least): where they do not (95^3: 48 of
-// 64) the two kernels are faster, 93.3 us for the V-cycle against 96.6.
-inline bool rr_fits(int nc) {
-    const int cols = std::min((nc + 1 + 31) / 32 * 32, kRrMaxCols);
-    const int tiles_k = (nc + cols - 2) / (cols - 1);
-    return 8 * (nc + 1) >= 7 * tiles_k * cols;
+    residual_restrict_body<NN, BNAT, FIRST_X>(x, b, bc, bsc, xc, g, halfc, h2inv, inv_c, depth, blockIdx.x, blockIdx.y,
+                                              blockIdx.z);
 }
 
 // The shape of a residual_restrict launch: columns for the nc + 1 cells of a row where 128 reach, and the coarse
@@ -848,7 +841,7 @@ __device__ __forceinline__ void prolong_pass_split_body(const float* __restrict_
                                                         float* __restrict__ x1, const float* __restrict__ bs1, int nc,
                                                         int halfc, const Split& g, int bx, int by, int bz) {
     const int K = bx * BX + threadIdx.x;
-    const int J = by * BY + threadIdx.y;  // one of each a warp
+    const int J = by * (int)blockDim.y + threadIdx.y;  // one of each a warp
     const int I = bz;
     if (K > nc || J > nc) return;
     if (I > 0 && I + 1 < nc && J > 0 && J + 1 < nc)

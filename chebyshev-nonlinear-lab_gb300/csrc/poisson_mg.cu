@@ -518,7 +518,7 @@ void PoissonMG::cycle32(size_t l) {
     const Split gc = make_split(nc);
     // the finest level of an apply from an FP32 vector reads b = r32 itself (never copied, see apply)
     const bool nat = finest && in32_;
-    if (csplit && rr_fits(nc)) {
+    if (n == 255 || n == 127 || n == 63) {
         const RrShape sh = rr_shape(nc, ctx_.sm_count);
         const bool fx = first_fused32(l + 1);
         auto pick = [&](auto nn) {
@@ -528,9 +528,8 @@ void PoissonMG::cycle32(size_t l) {
         };
         auto k = n == 255 ? pick(std::integral_constant<int, 255>{})
                : n == 127 ? pick(std::integral_constant<int, 127>{})
-               : n == 63  ? pick(std::integral_constant<int, 63>{})
-                          : pick(std::integral_constant<int, 0>{});
-        launch_pdl(k, sh.grid, sh.block, 0, s, x, nat ? in32_ : b, C.b32.p, C.bs32.p, C.xs, g, nc, gc.half,
+                          : pick(std::integral_constant<int, 63>{});
+        launch_pdl(k, sh.grid, sh.block, 0, s, x, nat ? in32_ : b, C.b32.p, C.bs32.p, C.xs, g, gc.half,
                    (float)L.h2inv, (float)C.inv, sh.depth);
         ctx_.count_launch();
     } else {
@@ -552,11 +551,13 @@ void PoissonMG::cycle32(size_t l) {
     if (l == 0) coarse_cycle();
     else cycle32(l + 1);
     const dim3 cg((nc + 1 + BX - 1) / BX, (nc + 1 + BY - 1) / BY, nc + 1);
-    if (post_ > 0) {  // with the first post-smoothing pass
-        if (!csplit) launch_pdl(k_prolong_pass_split<false, 0>, cg, blk, 0, s, C.cur32, x, bs, nc, gc.half, g);
-        else if (n == 255) launch_pdl(k_prolong_pass_split<true, 255>, cg, blk, 0, s, C.cur32, x, bs, nc, gc.half, g);
-        else if (n == 127) launch_pdl(k_prolong_pass_split<true, 127>, cg, blk, 0, s, C.cur32, x, bs, nc, gc.half, g);
-        else launch_pdl(k_prolong_pass_split<true, 0>, cg, blk, 0, s, C.cur32, x, bs, nc, gc.half, g);
+    if (post_ > 0) {  // with the first post-smoothing pass; blocks of half the rows where the SMs outnumber them twice
+        const bool few = 2 * (size_t)cg.x * cg.y * cg.z <= (size_t)ctx_.sm_count;
+        const dim3 pb(BX, few ? BY / 2 : BY), pg(cg.x, few ? (nc + 1 + BY / 2 - 1) / (BY / 2) : cg.y, cg.z);
+        if (!csplit) launch_pdl(k_prolong_pass_split<false, 0>, pg, pb, 0, s, C.cur32, x, bs, nc, gc.half, g);
+        else if (n == 255) launch_pdl(k_prolong_pass_split<true, 255>, pg, pb, 0, s, C.cur32, x, bs, nc, gc.half, g);
+        else if (n == 127) launch_pdl(k_prolong_pass_split<true, 127>, pg, pb, 0, s, C.cur32, x, bs, nc, gc.half, g);
+        else launch_pdl(k_prolong_pass_split<true, 0>, pg, pb, 0, s, C.cur32, x, bs, nc, gc.half, g);
     } else {
         if (csplit) launch_pdl(k_prolong_split<true>, cg, blk, 0, s, C.cur32, x, nc, gc.half, n, g.half);
         else launch_pdl(k_prolong_split<false>, cg, blk, 0, s, C.cur32, x, nc, gc.half, n, g.half);
