@@ -122,30 +122,30 @@ __global__ void __launch_bounds__(BX* BY) k_bprolong_pass(MgPool C, MgPool F, co
                                      blockIdx.y, blockIdx.z - q * (nc + 1));
 }
 
-// 31^3 and below of every grid of the 31^3 pool: a cluster of 8 CTAs a grid (mg_chain.cuh).  The first top0 grids
+// 31^3 and below of every grid of the 31^3 pool: a cluster of 32 / PL CTAs a grid (mg_chain.cuh).  The first top0 grids
 // take b from the pool and leave x there; the others are their instances' finest level: b is their basis vector (u +
 // (q - top0) N) and x their preconditioned vector (z + ...).  SHIFT (Jacobian-aware levels): level m's coefficients
 // of grid q are at io.c[m] + q n_m^3.
-template <bool SHIFT>
+template <bool SHIFT, int PL>
 __global__ void __launch_bounds__(kChainThreads, 1) k_bchain(MgPool P, const int* __restrict__ act, int top0,
                                                              const float* __restrict__ u, float* __restrict__ z,
                                                              const __grid_constant__ ChainIo io) {
-    using K = Chain32<SHIFT>;
+    using K = Chain32<SHIFT, PL>;
     using L31 = typename K::L31;
     constexpr long long N = 31 * 31 * 31;
-    const int rank = (int)cooperative_groups::this_cluster().block_rank(), my = min(4, 31 - 4 * rank);
+    const int rank = (int)cooperative_groups::this_cluster().block_rank(), my = min(PL, 31 - PL * rank);
     chain_clear<L31>();
     if (rank == 0) chain_clear_below31<K>();
     cooperative_groups::this_cluster().sync();
     pdl_wait();
     pdl_trigger();
-    const int q = blockIdx.x / kChainCluster;
+    const int q = blockIdx.x / (32 / PL);
     if (!pool_active(P, act, q)) return;  // (the whole cluster)
     const bool finest = q >= top0;
     chain_load_top<L31>(finest ? kChainSame : kChainSplit, io.half, finest ? u + (q - top0) * N : P.b + q * P.sb, my, rank);
     if (rank == 0) chain_coefs<K, SHIFT>(io, q);
     __syncthreads();
-    chain_cycle31<SHIFT>(io, SHIFT ? io.c[3] + q : nullptr, my, rank);
+    chain_cycle31<SHIFT, PL>(io, SHIFT ? io.c[3] + q : nullptr, my, rank);
     chain_store_top<L31>(io.half, finest ? nullptr : P.x + q * P.sx, finest ? z + (q - top0) * N : nullptr, nullptr, my,
                          rank);
     cooperative_groups::this_cluster().sync();

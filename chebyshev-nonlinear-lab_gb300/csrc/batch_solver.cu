@@ -354,7 +354,26 @@ struct BatchSolver::Impl {
         }
     };
     std::vector<std::unique_ptr<Pool>> pools;  // sizes n_max ... 15 (the last one is the tail)
+    using ChainKernel = void (*)(MgPool, const int*, int, const float*, float*, ChainIo);
+    ChainKernel chain_kern = nullptr;
     size_t chain_smem = 0;
+    int chain_cluster = 0;
+    template <bool SHIFT> void plan_chain();
+    cudaLaunchConfig_t chain_config(int grids, int cluster, size_t smem, cudaLaunchAttribute (&attr)[2]) const {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(grids * cluster));
+        cfg.blockDim = dim3(kChainThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = ctx.stream;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)cluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        return cfg;
+    }
     // Jacobian-aware tail (kp.coarse_jacobian): the coefficient c = lambda e^u of each pool grid below the
     // finest pool (natural layout, grid q at q s^3), and of the tail's levels 7, 3, 1 (grid q of the last pool)
     bool jac_tail = false;
@@ -573,10 +592,49 @@ void BatchSolver::Impl::alloc_state() {
         ctail[2].resize((size_t)Kt);
     }
     // 31^3 and below of every instance: one cluster each
-    chain_smem = (jac_tail ? Chain32<true>::TOTAL : Chain32<false>::TOTAL) * sizeof(float);
-    const int lim = jac_tail ? set_dynamic_smem_limit(ctx, k_bchain<true>) : set_dynamic_smem_limit(ctx, k_bchain<false>);
-    if (chain_smem > (size_t)lim) throw Status(NUMA_GPU_ERR_NOT_SUPPORTED, "batched multigrid exceeds shared memory");
+    if (jac_tail) plan_chain<true>();
+    else plan_chain<false>();
+    // The kernels around the chain read neighbours through L1, and an SM keeps the chain's division (28 KB of L1 beside
+    // 227 KB of shared memory) for them unless told otherwise: the 127^3 passes of 128 instances take 128 us with it
+    // and 120 with this, the batch 43.8 and 42.1 ms.
+    auto prefer_l1 = [](auto... kern) {
+        (cudaFuncSetAttribute(reinterpret_cast<const void*>(kern), cudaFuncAttributePreferredSharedMemoryCarveout,
+                              cudaSharedmemCarveoutMaxL1), ...);
+        cudaGetLastError();
+    };
+    prefer_l1(k_bpass<kPassFull, 4, 255>, k_bpass<kPassFull, 4, 127>, k_bpass<kPassFull, 4, 63>, k_bpass<kPassFull, 4, 0>,
+              k_bpass<kPassFull, 1, 0>, k_bpass<kPassLastZ, 4, 255>, k_bpass<kPassLastZ, 4, 127>,
+              k_bpass<kPassLastZ, 4, 0>, k_bpass<kPassLastZ, 1, 0>, k_bprolong_pass, k_bresidual, k_brestrict<true>,
+              k_brestrict<false>, k_bjvp32f, k_bscale_in<true>, k_brestrict_coef);
     ctx.sync();
+}
+
+// The cluster of the 31^3 pool's grids: 8 CTAs of 4 planes, or 4 of 8 planes where those take fewer waves.  A CTA has
+// an SM to itself, so 152 SMs run some 18 clusters of 8 or 36 of 4 at a time, and a wave of the smaller ones takes a
+// tenth longer.  128 grids: 273 us a V-cycle in clusters of 8, 139 in clusters of 4; 32 grids 77 and 36.
+template <bool SHIFT>
+void BatchSolver::Impl::plan_chain() {
+    const int K = pools[pools.size() - 2]->K;
+    long long best = 0;
+    auto consider = [&](ChainKernel kern, size_t smem, int cluster, int cost) {
+        if (smem > (size_t)set_dynamic_smem_limit(ctx, kern)) return;
+        cudaLaunchAttribute attr[2];
+        const cudaLaunchConfig_t cfg = chain_config(K, cluster, smem, attr);
+        int active = 0;
+        if (cudaOccupancyMaxActiveClusters(&active, kern, &cfg) != cudaSuccess || active < 1) {
+            cudaGetLastError();
+            return;
+        }
+        const long long t = (long long)cost * ((K + active - 1) / active);
+        if (best && t >= best) return;
+        best = t;
+        chain_kern = kern;
+        chain_cluster = cluster;
+        chain_smem = smem;
+    };
+    consider(k_bchain<SHIFT, 4>, Chain32<SHIFT, 4>::TOTAL * sizeof(float), 8, 10);
+    consider(k_bchain<SHIFT, 8>, Chain32<SHIFT, 8>::TOTAL * sizeof(float), 4, 11);
+    if (!best) throw Status(NUMA_GPU_ERR_NOT_SUPPORTED, "batched multigrid exceeds shared memory");
 }
 
 void BatchSolver::Impl::build_tables() {
@@ -775,21 +833,9 @@ void BatchSolver::Impl::vcycle(int j) {
             for (int m2 = 0; m2 < 3; ++m2) io.c[m2 + 1] = ctail[m2].p;
         }
         const long long off = P.cls >= 0 ? cls[P.cls].off0 : 0;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)P.K * kChainCluster);
-        cfg.blockDim = dim3(kChainThreads);
-        cfg.dynamicSmemBytes = chain_smem;
-        cfg.stream = s;
         cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = kChainCluster;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 2;
-        NUMA_CUDA(cudaLaunchKernelEx(&cfg, jac_tail ? k_bchain<true> : k_bchain<false>, P.view(), act, P.top0, u + off,
-                                     zout + off, io));
+        const cudaLaunchConfig_t cfg = chain_config(P.K, chain_cluster, chain_smem, attr);
+        NUMA_CUDA(cudaLaunchKernelEx(&cfg, chain_kern, P.view(), act, P.top0, u + off, zout + off, io));
         ctx.count_launch();
     }
     // up: prolongation and post-smoothing; the finest level of each instance writes z_j

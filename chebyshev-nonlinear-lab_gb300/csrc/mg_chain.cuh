@@ -255,27 +255,30 @@ __device__ __noinline__ void chain_restrict(int my, int rank) {
     }
     chain_sync<F::BAR>();
     constexpr int NC = C::N, planes = F::WIDE ? F::PL / 2 : NC;
-    const int t = threadIdx.x, I = t / (NC * NC), r = t - I * NC * NC, J = r / NC, K = r - J * NC;
-    const int Ig = F::WIDE ? rank * planes + I : I;
-    static_assert(planes * NC * NC <= kChainThreads);
-    if (I < planes && Ig < NC) {
-        // padded index of fine point (2I, 2J, 2K): odd, so offset d has parity (1 + d) & 1
-        const T* R = chain_base<T>() + OR + ((((2 * I + 1) * F::M + 2 * J + 1) * F::M + 2 * K + 1) >> 1);
-        constexpr T w[3] = {T(0.25), T(0.5), T(0.25)};
-        T acc = zero<T>();
+    constexpr int rounds = (planes * NC * NC + kChainThreads - 1) / kChainThreads;
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
+    for (int round = 0; round < rounds; ++round) {
+        const int t = threadIdx.x + round * kChainThreads, I = t / (NC * NC), r = t - I * NC * NC, J = r / NC, K = r - J * NC;
+        const int Ig = F::WIDE ? rank * planes + I : I;
+        if (I < planes && Ig < NC) {
+            // padded index of fine point (2I, 2J, 2K): odd, so offset d has parity (1 + d) & 1
+            const T* R = chain_base<T>() + OR + ((((2 * I + 1) * F::M + 2 * J + 1) * F::M + 2 * K + 1) >> 1);
+            constexpr T w[3] = {T(0.25), T(0.5), T(0.25)};
+            T acc = zero<T>();
 #pragma unroll
-            for (int b = 0; b < 3; ++b)
+            for (int a = 0; a < 3; ++a)
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const int d = (a * F::M + b) * F::M + c;
-                    acc = fma_t(w[a] * w[b] * w[c], R[((1 + d) & 1) * F::H + ((1 + d) >> 1)], acc);
-                }
-        const int P = ((Ig + 1) * C::M + J + 1) * C::M + K + 1;
-        T* B = chain_base<T>() + C::OB + (P & 1) * C::H + (P >> 1);
-        if constexpr (F::WIDE) chain_store(chain_addr(B, 0), acc);
-        else *B = acc;
+                for (int b = 0; b < 3; ++b)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const int d = (a * F::M + b) * F::M + c;
+                        acc = fma_t(w[a] * w[b] * w[c], R[((1 + d) & 1) * F::H + ((1 + d) >> 1)], acc);
+                    }
+            const int P = ((Ig + 1) * C::M + J + 1) * C::M + K + 1;
+            T* B = chain_base<T>() + C::OB + (P & 1) * C::H + (P >> 1);
+            if constexpr (F::WIDE) chain_store(chain_addr(B, 0), acc);
+            else *B = acc;
+        }
     }
     chain_sync<F::BAR>();
 }
@@ -286,7 +289,7 @@ template <class F, class C, int OR>
 __device__ __noinline__ void chain_prolong(int my, int rank) {
     using T = typename F::T;
     constexpr int NC1 = C::N + 1, cellp = F::WIDE ? F::PL / 2 : NC1;
-    static_assert(cellp * NC1 * NC1 <= kChainThreads);
+    constexpr int rounds = (cellp * NC1 * NC1 + kChainThreads - 1) / kChainThreads;
     const T* XC = chain_base<T>() + C::OX;
     constexpr int HS = F::WIDE ? ((F::PL / 2 + 1) * C::M2 + 2) / 2 : C::H;
     const int t = threadIdx.x;
@@ -303,32 +306,35 @@ __device__ __noinline__ void chain_prolong(int my, int rank) {
         XC = dst;
         __syncthreads();
     }
-    const int I = t / (NC1 * NC1), r = t - I * NC1 * NC1, J = r / NC1, K = r - J * NC1;
-    if (I < cellp && 2 * I < my) {
-        const int Pc = (I * C::M + J) * C::M + K, p0 = Pc & 1;
-        const T* even = XC + p0 * HS + (Pc >> 1);              // even offsets d at d / 2
-        const T* oddp = XC + (1 - p0) * HS + (Pc >> 1) + p0;   // odd ones at (d - 1) / 2
-        T v[8];
 #pragma unroll
-        for (int h = 0; h < 8; ++h) {
-            const int d = ((h >> 2) * C::M + ((h >> 1) & 1)) * C::M + (h & 1);
-            v[h] = (d & 1) ? oddp[(d - 1) / 2] : even[d / 2];
-        }
-        T* X = chain_base<T>() + F::OX;
-        const int P = (((2 * I + 1) * F::M + 2 * J + 1) * F::M + 2 * K + 1) >> 1;  // odd: parity 1 is colour 0
-        const bool in[3] = {2 * I + 1 < my, J < C::N, K < C::N};
+    for (int round = 0; round < rounds; ++round) {
+        const int tc = t + round * kChainThreads, I = tc / (NC1 * NC1), r = tc - I * NC1 * NC1, J = r / NC1, K = r - J * NC1;
+        if (I < cellp && 2 * I < my) {
+            const int Pc = (I * C::M + J) * C::M + K, p0 = Pc & 1;
+            const T* even = XC + p0 * HS + (Pc >> 1);              // even offsets d at d / 2
+            const T* oddp = XC + (1 - p0) * HS + (Pc >> 1) + p0;   // odd ones at (d - 1) / 2
+            T v[8];
 #pragma unroll
-        for (int f = 0; f < 8; ++f) {
-            const int a = f >> 2, b = (f >> 1) & 1, c = f & 1;
-            if ((a + b + c) & 1) continue;
-            const T w = (a ? T(1) : T(0.5)) * (b ? T(1) : T(0.5)) * (c ? T(1) : T(0.5));
-            T acc = zero<T>();
+            for (int h = 0; h < 8; ++h) {
+                const int d = ((h >> 2) * C::M + ((h >> 1) & 1)) * C::M + (h & 1);
+                v[h] = (d & 1) ? oddp[(d - 1) / 2] : even[d / 2];
+            }
+            T* X = chain_base<T>() + F::OX;
+            const int P = (((2 * I + 1) * F::M + 2 * J + 1) * F::M + 2 * K + 1) >> 1;  // odd: parity 1 is colour 0
+            const bool in[3] = {2 * I + 1 < my, J < C::N, K < C::N};
 #pragma unroll
-            for (int h = 0; h < 8; ++h)
-                if (!((a && !(h >> 2)) || (b && !((h >> 1) & 1)) || (c && !(h & 1)))) acc = fma_t(w, v[h], acc);
-            const int i = P + ((a * F::M + b) * F::M + c) / 2;
-            if ((!a || in[0]) && (!b || in[1]) && (!c || in[2]))
-                chain_put<F, 1>(X, i, 2 * I + a, my, rank, X[F::H + i] + acc);
+            for (int f = 0; f < 8; ++f) {
+                const int a = f >> 2, b = (f >> 1) & 1, c = f & 1;
+                if ((a + b + c) & 1) continue;
+                const T w = (a ? T(1) : T(0.5)) * (b ? T(1) : T(0.5)) * (c ? T(1) : T(0.5));
+                T acc = zero<T>();
+#pragma unroll
+                for (int h = 0; h < 8; ++h)
+                    if (!((a && !(h >> 2)) || (b && !((h >> 1) & 1)) || (c && !(h & 1)))) acc = fma_t(w, v[h], acc);
+                const int i = P + ((a * F::M + b) * F::M + c) / 2;
+                if ((!a || in[0]) && (!b || in[1]) && (!c || in[2]))
+                    chain_put<F, 1>(X, i, 2 * I + a, my, rank, X[F::H + i] + acc);
+            }
         }
     }
     chain_sync<F::BAR>();
@@ -419,11 +425,11 @@ __device__ __noinline__ void chain_store_top(int half, float* x_split, void* x_n
     }
 }
 
-// The level tables: FP32 with 31^3 on top, FP64 with 15^3.
-template <bool SHIFT>
+// The level tables: FP32 with 31^3 on top (PL planes a CTA), FP64 with 15^3.
+template <bool SHIFT, int PL = 4>
 struct Chain32 {
     using T = float;
-    using L31 = ChainLv<float, 31, 4, true, kBarCluster, false, 0>;
+    using L31 = ChainLv<float, 31, PL, true, kBarCluster, false, 0>;
     using L15 = ChainLv<float, 15, 15, false, kBarCta, SHIFT, L31::END>;
     using L7 = ChainLv<float, 7, 7, false, kBarGroup, SHIFT, L15::END>;
     using L3 = ChainLv<float, 3, 3, false, kBarWarp, SHIFT, L7::END>;
@@ -478,10 +484,10 @@ __device__ __forceinline__ void chain_coefs(const ChainIo& io, size_t q) {
     }
 }
 
-// The cycle from 31^3 (b loaded) on a cluster of 8, in FP32.
-template <bool SHIFT>
+// The cycle from 31^3 (b loaded) on a cluster, in FP32.
+template <bool SHIFT, int PL = 4>
 __device__ __forceinline__ void chain_cycle31(const ChainIo& io, const float* c1, int my, int rank) {
-    using K = Chain32<SHIFT>;
+    using K = Chain32<SHIFT, PL>;
     using L31 = typename K::L31;
     chain_sweeps<L31>(my, rank, 2 * io.pre, 0, true);
     chain_restrict<L31, typename K::L15, K::OR>(my, rank);
