@@ -15,7 +15,7 @@
 // together (blockIdx.z = field); programmatic dependent launch; the levels below the finest in one CUDA graph; the
 // levels of 15 < n <= 127 in two tiled kernels each, on as many SMs as there are, where a step is a block barrier; and
 // the levels below in one CTA a field, in shared memory (k_hmg_tail).  The Burgers solve at 255^2 went from 17.5 to
-// 3.25 ms; a cycle of both fields is 82 us there (110 with 63^2 and 127^2 launched pass by pass and 31^2 in the tail):
+// 3.2 ms; a cycle of both fields is 82 us there (110 with 63^2 and 127^2 launched pass by pass and 31^2 in the tail):
 // 30 of them the finest level's 11 launches, 16 the tail (steps bound by the latency of their nine dependent FP64
 // operations), 11 each the levels between.
 #include <cmath>
