@@ -603,8 +603,9 @@ void BatchSolver::Impl::alloc_state() {
         cudaGetLastError();
     };
     prefer_l1(k_bpass<kPassFull, 4, 255>, k_bpass<kPassFull, 4, 127>, k_bpass<kPassFull, 4, 63>, k_bpass<kPassFull, 4, 0>,
-              k_bpass<kPassFull, 1, 0>, k_bpass<kPassLastZ, 4, 255>, k_bpass<kPassLastZ, 4, 127>,
-              k_bpass<kPassLastZ, 4, 0>, k_bpass<kPassLastZ, 1, 0>, k_bprolong_pass, k_bresidual, k_brestrict<true>,
+              k_bpass<kPassFull, 1, 0>, k_bpass<kPassLastZ, 4, 127>, k_bpass<kPassLastZ, 4, 63>,
+              k_bpass<kPassLastZ, 4, 0>, k_bpass<kPassLastZ, 1, 0>, k_bprolong_pass<127>, k_bprolong_pass<63>,
+              k_bprolong_pass<0>, k_bresidual, k_brestrict<true>,
               k_brestrict<false>, k_bjvp32f, k_bscale_in<true>, k_brestrict_coef);
     ctx.sync();
 }
@@ -751,7 +752,8 @@ void BatchSolver::Impl::vcycle(int j) {
             const dim3 grid(grid0.x, grid0.y, cnt * zch);
             float* zq = z32 ? z32 + (long long)(a - g0) * zs : nullptr;
             if (mode == kPassLastZ) {
-                if (four && n == 63) launch_pdl(k_bpass<kPassLastZ, 4, 63>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
+                if (n == 127) launch_pdl(k_bpass<kPassLastZ, 4, 127>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
+                else if (four && n == 63) launch_pdl(k_bpass<kPassLastZ, 4, 63>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
                 else if (four) launch_pdl(k_bpass<kPassLastZ, 4, 0>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
                 else launch_pdl(k_bpass<kPassLastZ, 1, 0>, grid, blk, 0, s, V, act, a, zch, g, c, zq, zs);
             } else {
@@ -853,7 +855,9 @@ void BatchSolver::Impl::vcycle(int j) {
             Cw.x += (long long)a * CV.sx;
             Cw.inst += a;
             const dim3 cg((nc + 1 + BX - 1) / BX, (nc + 1 + BY - 1) / BY, cnt * (nc + 1));
-            launch_pdl(k_bprolong_pass, cg, blk, 0, s, Cw, Fw, act, nc, gc.half, g);
+            if (n == 127) launch_pdl(k_bprolong_pass<127>, cg, blk, 0, s, Cw, Fw, act, nc, gc.half, g);
+            else if (n == 63) launch_pdl(k_bprolong_pass<63>, cg, blk, 0, s, Cw, Fw, act, nc, gc.half, g);
+            else launch_pdl(k_bprolong_pass<0>, cg, blk, 0, s, Cw, Fw, act, nc, gc.half, g);
             ctx.count_launch();
         });
         for (int sw = 0; sw < post; ++sw) {
