@@ -552,16 +552,6 @@ struct Context {
     Context& operator=(const Context&) = delete;
 
     void sync();
-    // Announces that src[0..count) will be fetched: the kernel whose reduction writes src[count - 1] takes the
-    // announcement (take) and leaves the values for the host itself, instead of a kernel of its own for that.
-    void expect(const double* src, int count);
-    HostOut take(const double* out) {
-        if (!armed.dst || out != armed.src + armed.count - 1) return {};
-        taken = true;
-        return armed;
-    }
-    HostOut armed;
-    bool taken = false;
     // Copies count device doubles to host memory and waits for them (and for all earlier work on the stream).
     void fetch(const double* dsrc, int count, double* host);
     double fetch1(const double* dsrc) {
@@ -569,12 +559,63 @@ struct Context {
         fetch(dsrc, 1, &v);
         return v;
     }
+    // For a kernel whose reduction writes *out: where to leave the announced scalars (Announced), if *out is the last
+    // of them.
+    HostOut take(const double* out) {
+        if (!armed.dst || out != armed.src + armed.count - 1) return {};
+        taken = true;
+        return armed;
+    }
+    // Where the next scalars go, under a new sequence number; and the wait for that number.
+    HostOut host_out(const double* src, int count);
+    void wait_published(unsigned long long seq, int count, double* host);
+    HostOut armed;       // the announcement in force (dst null: none), and whether a kernel has taken it
+    bool taken = false;
     double* scalar(int slot) { return d_scalars + slot; }
     // Number of blocks of kRedThreads threads for a grid-stride reduction over N elements.
     unsigned red_grid(size_t N) const;
     void count_launch(unsigned n = 1) { launches += n; }
     void check_launch(const char* what);
 };
+
+// Announces that src[0..count) will be fetched: the kernel whose reduction writes src[count - 1] (Context::take) leaves
+// the values for the host itself, instead of a kernel of its own for that.  fetch then waits for that kernel: for all
+// work before it on the stream, not for what was queued behind it.  The announcement ends with the object, so that none
+// outlives an exception between the two, and is void once another one or a plain fetch has come between.
+class Announced {
+public:
+    Announced(Context& c, const double* src, int count) : c_(c), src_(src), count_(count) {
+        c_.armed = c_.host_out(src, count);
+        c_.taken = false;
+        seq_ = c_.armed.seq;
+    }
+    ~Announced() { end(); }
+    Announced(const Announced&) = delete;
+    Announced& operator=(const Announced&) = delete;
+    void fetch(double* host) {
+        const bool left = c_.armed.seq == seq_ && c_.taken;
+        end();
+        if (left) c_.wait_published(seq_, count_, host);
+        else c_.fetch(src_, count_, host);
+    }
+    double fetch1() {
+        double v;
+        fetch(&v);
+        return v;
+    }
+
+private:
+    void end() {
+        if (c_.armed.seq != seq_) return;
+        c_.armed = HostOut{};
+        c_.taken = false;
+    }
+    Context& c_;
+    const double* src_;
+    int count_;
+    unsigned long long seq_;
+};
+
 // Programmatic dependent launch.  A kernel launched by launch_pdl may be scheduled while its
 // predecessor on the stream is still running; it must call pdl_wait() before it touches memory
 // (griddepcontrol.wait returns once every prerequisite grid has completed and its writes are

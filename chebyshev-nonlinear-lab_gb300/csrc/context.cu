@@ -72,29 +72,27 @@ __global__ void k_publish(HostOut h) {
     host_publish(h, threadIdx.x, blockDim.x);
 }
 
-void Context::expect(const double* src, int count) {
-    taken = false;
-    armed = HostOut{};
-    if (count <= 0 || count > kNumScalars) return;
-    armed = HostOut{h_scalars_dev, reinterpret_cast<unsigned long long*>(h_scalars_dev + kNumScalars), ++fetch_seq, src,
-                    count};
+HostOut Context::host_out(const double* src, int count) {
+    if (count < 1 || count > kNumScalars) throw Status(NUMA_GPU_ERR_INVALID_ARGUMENT, "fetch too large");
+    return HostOut{h_scalars_dev, reinterpret_cast<unsigned long long*>(h_scalars_dev + kNumScalars), ++fetch_seq, src,
+                   count};
 }
 
 // A scalar the host decides on (a norm, a Hessenberg column) is read back dozens of times a solve, each time
 // with the GPU idle until the host has launched what follows.  A copy and a stream synchronisation take ~12 us; a
 // one-block kernel that writes mapped host memory, watched by the host, about half of that; the reduction that
-// forms the scalar writing it there itself (expect), another ~3 us less.
+// forms the scalar writing it there itself (Announced), another ~3 us less.
 void Context::fetch(const double* dsrc, int count, double* host) {
     if (count <= 0) return;
-    if (count > kNumScalars) throw Status(NUMA_GPU_ERR_INVALID_ARGUMENT, "fetch too large");
-    if (!(taken && armed.src == dsrc && armed.count == count)) {
-        expect(dsrc, count);
-        launch_pdl(k_publish, 1, 64, 0, stream, armed);
-        count_launch();
-    }
-    const unsigned long long seq = armed.seq;
     armed = HostOut{};
     taken = false;
+    const HostOut h = host_out(dsrc, count);
+    launch_pdl(k_publish, 1, 64, 0, stream, h);
+    count_launch();
+    wait_published(h.seq, count, host);
+}
+
+void Context::wait_published(unsigned long long seq, int count, double* host) {
     auto* word = reinterpret_cast<unsigned long long*>(h_scalars + kNumScalars);
     const auto arrived = [&] { return __atomic_load_n(word, __ATOMIC_ACQUIRE) == seq; };
     for (unsigned spins = 0; !arrived(); ++spins) {

@@ -300,12 +300,12 @@ struct SolveState {
         return p.jvp_precision == NUMA_GPU_FP32 && p.jvp_mode == NUMA_GPU_DERIV_ANALYTIC ? f.f32_of_cache(cx) : nullptr;
     }
     double eval_trial() {
-        ctx.expect(ctx.scalar(kSlotNormF), 1);
+        Announced norm(ctx, ctx.scalar(kSlotNormF), 1);
         {
             Timers::Scope s(&timers, kT_F);
             f.eval(xn, Fn, cn, ctx.scalar(kSlotNormF));
         }
-        return ctx.fetch1(ctx.scalar(kSlotNormF));
+        return norm.fetch1();
     }
     void accept() {
         std::swap(x, xn);

@@ -744,6 +744,12 @@ void Gmres::precond_apply(Precond* M, const double* r, double* z) {
     else dev_copy(ctx_, r, z, N_);
 }
 
+double Gmres::norm(const double* v, double* slot) {
+    Announced a(ctx_, slot, 1);
+    dev_norm2(ctx_, v, N_, slot);
+    return a.fetch1();
+}
+
 // Leaves H[0..j][j] in hcol[0..j] and ||w|| in hcol[j+1]; w is orthogonalised in place.
 void Gmres::arnoldi_mgs(size_t j, double* w) {
     double* hcol = ctx_.scalar(kSlotGmresH);
@@ -827,9 +833,7 @@ GmresResult Gmres::solve_lazy(LinearOp& A, Precond* M, const double* b, double* 
     double* sig2 = ctx_.scalar(kSlotGmresSig2);
     double bnorm = o.bnorm;
     if (bnorm < 0.0) {
-        ctx_.expect(sl, 1);
-        dev_norm2(ctx_, b, N, sl);
-        bnorm = ctx_.fetch1(sl);
+        bnorm = norm(b, sl);
     }
     if (bnorm == 0.0) {
         dev_fill(ctx_, x, 0.0, N);
@@ -899,9 +903,7 @@ GmresResult Gmres::solve_lazy(LinearOp& A, Precond* M, const double* b, double* 
             v0 = r_init;
             given = false;
             first = false;
-            ctx_.expect(sl, 1);
-            dev_norm2(ctx_, v0, N, sl);
-            beta = ctx_.fetch1(sl);
+            beta = norm(v0, sl);
         } else if (first) {
             v0 = b;
             first = false;
@@ -916,9 +918,7 @@ GmresResult Gmres::solve_lazy(LinearOp& A, Precond* M, const double* b, double* 
             launch_pdl(k_sub, eg, 256, 0, ctx_.stream, b, w_.p, r_.p, N);
             ctx_.count_launch();
             v0 = r_.p;
-            ctx_.expect(sl, 1);
-            dev_norm2(ctx_, v0, N, sl);
-            beta = ctx_.fetch1(sl);
+            beta = norm(v0, sl);
         }
         res.rel_res = beta / bnorm;
         if (res.rel_res <= o.rtol) {
@@ -970,7 +970,7 @@ GmresResult Gmres::solve_lazy(LinearOp& A, Precond* M, const double* b, double* 
             }
             ++res.matvecs;
             const int cnt = (int)(j + 1);
-            ctx_.expect(sl, (int)(j + 2));
+            Announced column(ctx_, sl, (int)(j + 2));
             float* unext = v32 ? V32_.p + (j + 1) * N : nullptr;
             if (v32 && !two_pass) {
                 cgs_dots_df(ctx_, cnt, W32_.p, u0, V32_.p, N, sl);
@@ -993,7 +993,7 @@ GmresResult Gmres::solve_lazy(LinearOp& A, Precond* M, const double* b, double* 
                 cgs_update<2>(ctx_, cnt, w_.p, v0, V_.p, N, h2, sig2, sl + j + 1, V_.p + (j + 1) * N, sig2 + j + 1);
             }
             ctx_.check_launch("arnoldi (lazy cgs)");
-            ctx_.fetch(sl, (int)(j + 2), col.data());
+            column.fetch(col.data());
             if (two_pass) ctx_.fetch(h2, (int)(j + 1), col2.data());
             for (size_t i = 0; i <= j; ++i) H[i][j] = sig[j] * sig[i] * col[i];
             // the second pass' coefficients: on sigma_j w~ (FP32 basis) or on w~ itself
@@ -1085,9 +1085,7 @@ GmresResult Gmres::solve(LinearOp& A, Precond* M, const double* b, double* x, co
     if (save) save->clear();
 
     double* sl = ctx_.scalar(kSlotGmresH);
-    ctx_.expect(sl, 1);
-    dev_norm2(ctx_, b, N, sl);
-    const double bnorm = ctx_.fetch1(sl);
+    const double bnorm = norm(b, sl);
     if (bnorm == 0.0) {
         dev_fill(ctx_, x, 0.0, N);
         res.converged = true;
@@ -1140,9 +1138,7 @@ GmresResult Gmres::solve(LinearOp& A, Precond* M, const double* b, double* x, co
             ctx_.count_launch();
             rv = r_.p;
         }
-        ctx_.expect(sl, 1);
-        dev_norm2(ctx_, rv, N, sl);
-        const double beta = ctx_.fetch1(sl);
+        const double beta = norm(rv, sl);
         res.rel_res = beta / bnorm;
         if (res.rel_res <= o.rtol) {
             res.converged = true;
@@ -1164,7 +1160,7 @@ GmresResult Gmres::solve(LinearOp& A, Precond* M, const double* b, double* x, co
             ++res.precs;
             A.apply(zj, w_.p);
             ++res.matvecs;
-            ctx_.expect(sl, (int)(j + 2));
+            Announced column(ctx_, sl, (int)(j + 2));
             if (cgs2) {
                 arnoldi_cgs2(j, w_.p);
             } else if (cgs1) {
@@ -1175,7 +1171,7 @@ GmresResult Gmres::solve(LinearOp& A, Precond* M, const double* b, double* x, co
             launch_pdl(k_div_dev, eg, 256, 0, ctx_.stream, (const double*)w_.p, (const double*)(sl + j + 1),
                        cgs1 || cgs2 ? nullptr : (const double*)ctx_.scalar(kSlotGmresRnorm), V_.p + (j + 1) * N, N);
             ctx_.count_launch();
-            ctx_.fetch(sl, (int)(j + 2), col.data());
+            column.fetch(col.data());
             if (cgs2) {
                 ctx_.fetch(ctx_.scalar(kSlotGmresH2), (int)(j + 1), col2.data());
                 for (size_t i = 0; i <= j; ++i) col[i] += col2[i];
@@ -1229,7 +1225,7 @@ GmresResult Gmres::solve(LinearOp& A, Precond* M, const double* b, double* x, co
             ++res.precs;
             dev_axpy(ctx_, 1.0, z_.p, x, N);
         }
-        // (the pinned y buffer is next written after a later fetch has synchronised the stream)
+        // (the pinned y buffer is next written after a later fetch, which waits for all work before it)
         ctx_.check_launch("gmres update");
         if (res.rel_res <= o.rtol) {
             res.converged = true;

@@ -623,6 +623,7 @@ public:
                                KrylovSpace* save = nullptr);
 
 private:
+    double norm(const double* v, double* slot);  // ||v||, through the device scalar slot
     void arnoldi_mgs(size_t j, double* w);
     void arnoldi_cgs2(size_t j, double* w);
     void arnoldi_cgs1(size_t j, double* w);
