@@ -533,6 +533,7 @@ void Bratu3D::eval_as(const double* x, int precision, double* out, double* norm_
     double* nrm = ctx_.scalar(kSlotTmp0);
     eval(x, out, cache.p, nrm);
     const double v = ctx_.fetch1(nrm);
+    ctx_.sync();
     if (norm_host) *norm_host = v;
     mixed_cache_ = keep;
 }

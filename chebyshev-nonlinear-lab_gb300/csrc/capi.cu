@@ -464,6 +464,7 @@ int numa_gpu_vec_dot(const numa_gpu_vec* a, const numa_gpu_vec* b, double* out) 
         }
         dev_dot(c, a->d, b->d, a->n, c.scalar(kSlotTmp0));
         *out = c.fetch1(c.scalar(kSlotTmp0));
+        c.sync();  // (the fetch waits for the value, not for the kernel that left it)
     });
 }
 
@@ -477,6 +478,7 @@ int numa_gpu_vec_norm2(const numa_gpu_vec* a, double* out) {
         }
         dev_norm2(c, a->d, a->n, c.scalar(kSlotTmp0));
         *out = c.fetch1(c.scalar(kSlotTmp0));
+        c.sync();  // (the fetch waits for the value, not for the kernel that left it)
     });
 }
 

@@ -552,7 +552,8 @@ struct Context {
     Context& operator=(const Context&) = delete;
 
     void sync();
-    // Copies count device doubles to host memory and waits for them (and for all earlier work on the stream).
+    // Copies count device doubles to host memory and waits for them (and for all earlier work on the stream; the
+    // kernel that leaves them may still be ending, so an entry point that promises an idle stream synchronises it).
     void fetch(const double* dsrc, int count, double* host);
     double fetch1(const double* dsrc) {
         double v;
