@@ -95,14 +95,26 @@ void Context::fetch(const double* dsrc, int count, double* host) {
 void Context::wait_published(unsigned long long seq, int count, double* host) {
     auto* word = reinterpret_cast<unsigned long long*>(h_scalars + kNumScalars);
     const auto arrived = [&] { return __atomic_load_n(word, __ATOMIC_ACQUIRE) == seq; };
+    bool yield = false;
     for (unsigned spins = 0; !arrived(); ++spins) {
+        if (spins < 1024) continue;
+        if (spins == 1024) {  // a wait of microseconds or more: as the caller has the device schedule its waits
+            unsigned flags = 0;
+            NUMA_CUDA(cudaGetDeviceFlags(&flags));
+            if ((flags & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync) {
+                sync();  // its writes are visible
+                break;
+            }
+            yield = (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleYield;
+        }
+        if (yield) std::this_thread::yield();
         if (spins < 32768 || (spins & 255)) continue;
         // a long wait: let other threads run, and look whether the stream has failed or ended
         std::this_thread::yield();
         const cudaError_t e = cudaStreamQuery(stream);
         if (e == cudaErrorNotReady) continue;
         NUMA_CUDA(e);
-        if (!arrived()) NUMA_CUDA(cudaStreamSynchronize(stream));  // ended: its writes are visible
+        if (!arrived()) sync();  // ended: its writes are visible
         break;
     }
     for (int i = 0; i < count; ++i) host[i] = h_scalars[i];

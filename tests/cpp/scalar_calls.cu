@@ -1,7 +1,9 @@
 // Calls that return a scalar to the host, seen from a program that shares the context's stream:
 //   idle      how often the stream still has work when vec_norm2, vec_dot or diag_eval returns (expected 0)
+//   blocking  with the device set to block its waiting threads: the share of a long wait that the thread spent running
 #include <cstdio>
 #include <cstring>
+#include <ctime>
 
 #include <cuda_runtime.h>
 
@@ -40,7 +42,41 @@ static int idle() {
     return 0;
 }
 
+static double seconds(clockid_t c) {
+    timespec t;
+    clock_gettime(c, &t);
+    return (double)t.tv_sec + 1e-9 * (double)t.tv_nsec;
+}
+
+static int blocking() {
+    if (cudaSetDeviceFlags(cudaDeviceScheduleBlockingSync) != cudaSuccess) return 1;
+    const size_t n = 127, N = n * n * n;
+    numa_gpu_ctx* ctx;
+    numa_gpu_vec *r, *z;
+    numa_gpu_mg* mg;
+    if (check(numa_gpu_ctx_create(0, &ctx), "ctx") || check(numa_gpu_vec_create(ctx, N, &r), "vec") ||
+        check(numa_gpu_vec_create(ctx, N, &z), "vec") || check(numa_gpu_mg_create(ctx, n, 2, 2, &mg), "mg"))
+        return 1;
+    double v, wall = 0.0, cpu = 0.0;
+    for (int rep = 0; rep < 2; ++rep) {  // the second is timed
+        for (int i = 0; i < 300; ++i)    // tens of milliseconds
+            if (check(numa_gpu_mg_apply(mg, r, z), "apply")) return 1;
+        wall = -seconds(CLOCK_MONOTONIC);
+        cpu = -seconds(CLOCK_THREAD_CPUTIME_ID);
+        if (check(numa_gpu_vec_norm2(z, &v), "norm2")) return 1;
+        cpu += seconds(CLOCK_THREAD_CPUTIME_ID);
+        wall += seconds(CLOCK_MONOTONIC);
+    }
+    std::printf("%g %g\n", cpu / wall, wall);
+    numa_gpu_mg_destroy(mg);
+    numa_gpu_vec_destroy(r);
+    numa_gpu_vec_destroy(z);
+    numa_gpu_ctx_destroy(ctx);
+    return 0;
+}
+
 int main(int argc, char** argv) {
     if (argc > 1 && !std::strcmp(argv[1], "idle")) return idle();
+    if (argc > 1 && !std::strcmp(argv[1], "blocking")) return blocking();
     return 2;
 }

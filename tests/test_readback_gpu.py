@@ -33,3 +33,10 @@ def test_scalar_calls_leave_the_stream_idle(lib_path, tmp_path):
     """Calls that return a scalar synchronise the context's stream: 2,000 each of a norm, an inner product and a
     residual norm leave no work on it."""
     assert _run(_program("scalar_calls", tmp_path), "idle") == [0, 0, 0]
+
+
+def test_waits_follow_the_device_schedule(lib_path, tmp_path):
+    """Where the program has the device block its waiting threads (cudaDeviceScheduleBlockingSync), a wait of
+    milliseconds for a norm leaves the core to others."""
+    share, wall = _run(_program("scalar_calls", tmp_path), "blocking")
+    assert wall > 2e-3 and share < 0.5
