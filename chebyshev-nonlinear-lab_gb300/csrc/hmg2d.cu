@@ -510,9 +510,12 @@ void HelmholtzMG2D::launch_tail(const double* b, double* x) {
     ctx_.check_launch("hmg2d tail");
 }
 
-// The levels below the finest touch only the hierarchy's own arrays: captured once, then one launch.
+// The levels below the finest touch only the hierarchy's own arrays: captured once, then one launch.  Inside a caller's
+// own capture of the stream their kernels go into that graph.
 void HelmholtzMG2D::coarse_cycle() {
-    if (tail_l_ == 1) {  // one kernel: no graph
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    NUMA_CUDA(cudaStreamIsCapturing(ctx_.stream, &cap));
+    if (tail_l_ == 1 || cap != cudaStreamCaptureStatusNone) {  // (or one kernel: no graph)
         cycle(1);
         return;
     }
