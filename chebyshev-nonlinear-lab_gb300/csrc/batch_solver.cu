@@ -475,7 +475,11 @@ BatchSolver::BatchSolver(Context& ctx, const numa_batch_instance* inst, size_t c
                                       (long long)(inst[u].n * inst[u].n * inst[u].n)});
         M.cls.back().count += 1;
     }
+    // the default block: at least eight blocks an SM where the batch is small (with more elements a block 32 instances of
+    // 31^3 and 63^3 made 100 blocks, and a Gram-Schmidt pass over four vectors took 79 us)
+    const long long fill = std::max<long long>(2048, M.T / (8LL * ctx.sm_count) / 1024 * 1024);
     M.tune = BatchTuning{};
+    M.tune.elems_per_block = (int)std::min<long long>(M.tune.elems_per_block, fill);
     M.alloc_state();
     M.build_tables();
 }
@@ -640,10 +644,7 @@ void BatchSolver::Impl::plan_chain() {
 
 void BatchSolver::Impl::build_tables() {
     // element-wise block table
-    // at least eight blocks an SM where the batch is small: at 32,768 elements a block 32 instances of 31^3 and 63^3
-    // made 100 blocks, and a Gram-Schmidt pass over four vectors took 79 us
-    const long long fill = std::max<long long>(2048, T / (8LL * ctx.sm_count) / 1024 * 1024);
-    const long long E = std::min<long long>(std::max(1024, tune.elems_per_block), fill);
+    const long long E = std::max(1024, tune.elems_per_block);
     std::vector<int> bi, b0(I), bn(I);
     std::vector<long long> bb, be;
     for (int t = 0; t < I; ++t) {

@@ -722,7 +722,7 @@ private:
 // element-wise passes (Gram-Schmidt, solution update, line-search step) covers.
 struct BatchTuning {
     int planes = 8;
-    int elems_per_block = 16384;
+    int elems_per_block = 16384;  // (a new solver takes fewer for a small batch)
 };
 
 // Many Bratu3D instances of uneven size (n = 2^k - 1, 31 ... 1023) and lambda solved together by

@@ -539,7 +539,10 @@ const char* numa_gpu_batch_last_error(void);
 typedef struct numa_gpu_bsolver numa_gpu_bsolver;
 typedef struct numa_batch_tuning {
     int32_t planes;          /* planes a thread marches in the residual and Jacobian stencils */
-    int32_t elems_per_block; /* elements a block of the element-wise passes covers */
+    int32_t elems_per_block; /* elements a block of the element-wise passes covers, and so a group of the
+                                partial sums of its instance's inner products: a new solver chooses it by
+                                the batch's total size, so the last bits of an instance's solution depend
+                                on the batch; with a value set here they depend on the instance alone */
     int32_t reserved[6];
 } numa_batch_tuning;
 int numa_gpu_bsolver_create(numa_gpu_ctx* ctx, const numa_batch_instance* inst, size_t count,
