@@ -252,8 +252,7 @@ __global__ void __launch_bounds__(kBX* kBY, 5) k_beval(const double* __restrict_
             p += plane;
         }
     }
-    __shared__ double sm[1][32];
-    block_sum<1>(acc, sm);
+    block_sum<1>(acc);
     if (threadIdx.x == 0 && threadIdx.y == 0)
         partials[C.pbase + ((size_t)(gq * C.zch + bz) * C.jb + blockIdx.y) * C.kb + blockIdx.x] = acc[0];
 }
@@ -341,8 +340,7 @@ constexpr int kCgsBlock = 8;  // basis vectors per fused Gram-Schmidt / update p
 // Block reduction of R sums to partials[b * R + r] (thread 0).
 template <int R>
 __device__ __forceinline__ void block_partials(double (&s)[R], double* __restrict__ partials) {
-    __shared__ double sm[R][32];
-    block_sum<R>(s, sm);
+    block_sum<R>(s);
     if (threadIdx.x == 0)
 #pragma unroll
         for (int r = 0; r < R; ++r) partials[(size_t)blockIdx.x * R + r] = s[r];
@@ -586,6 +584,7 @@ __global__ void __launch_bounds__(kEwThreads) k_bscale32(const double* __restric
 // Per-instance sums of block partials: out[t * ostride + ooff + r] = sum over the instance's partial slots
 // [p0[t], p0[t] + pn[t]) of partials[slot * R + r], for r < R <= 8.  One warp per instance; its lanes share out the
 // slots (in an order that depends on R and pn alone): one lane a result took 26 us for 130 slots.
+static_assert(kCgsBlock <= 8, "k_bsegsum: 32 lanes, four a result");
 __global__ void k_bsegsum(const double* __restrict__ partials, int R, const int* __restrict__ p0,
                           const int* __restrict__ pn, const int* __restrict__ act, int I, double* __restrict__ out,
                           int ostride, int ooff) {

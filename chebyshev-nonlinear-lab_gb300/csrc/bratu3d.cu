@@ -27,12 +27,12 @@ struct March {
 // Grid of (k tiles, j tiles, i chunks).  Chunks of 8 planes keep ~2M threads at n = 255; a fused
 // reduction takes 16 from n = 128 (its block sum, in FP64, is then shared by twice the points), and
 // more when it would exceed kMaxRedBlocks partials.  Smaller grids halve the chunk until there are four
-// blocks an SM (152 SMs): a march of 4 planes at 31^3 left four SMs in five idle and was bound by the latency of
+// blocks an SM: a march of 4 planes at 31^3 left four SMs in five idle and was bound by the latency of
 // its FP64 operations (the product from x 5.8 us, with one plane a thread 2.8; with c given 4.5 and 2.5).
-March march_shape(int n, bool reducing) {
+March march_shape(int n, bool reducing, int sm_count) {
     const int kb = (n + BX - 1) / BX, jb = (n + BY - 1) / BY;
     int ichunk = reducing && n >= 128 ? 16 : 8;
-    while (ichunk > 1 && (long)kb * jb * ((n + ichunk - 1) / ichunk) < 4 * 152) ichunk /= 2;
+    while (ichunk > 1 && (long)kb * jb * ((n + ichunk - 1) / ichunk) < 4L * sm_count) ichunk /= 2;
     if (reducing) {
         const long cols = (long)kb * jb;
         const long max_chunks = kMaxRedBlocks / cols;
@@ -129,8 +129,7 @@ __global__ void __launch_bounds__(BX* BY, C32 ? 5 : 1) k_eval(const double* __re
         }
     }
     if (NORM) {
-        __shared__ double sm[1][32];
-        block_sum<1>(acc, sm);
+        block_sum<1>(acc);
         grid_reduce_finish<1>(acc, red, [norm_out, norm_raw] __device__(const double(&t)[1]) {
             *norm_out = norm_raw ? t[0] : __dsqrt_rn(t[0]);  // raw: a piece's sum of squares
         }, host);
@@ -477,7 +476,7 @@ void Bratu3D::bind(const double*, const double* cache, int precision) {
 
 void Bratu3D::jvp_bound32(const float* v32, double* out) {
     if (bound_precision_ != NUMA_GPU_FP32) throw Status(NUMA_GPU_ERR_INVALID_ARGUMENT, "Bratu3D: no FP32 product bound");
-    March m = march_shape((int)n_, false);
+    March m = march_shape((int)n_, false, ctx_.sm_count);
     launch_pdl(k_jvp32f<double>, m.grid, dim3(BX, BY), 0, ctx_.stream, bound_c32_, v32, out, (int)n_, m.ichunk,
                (float)h2inv_);
     ctx_.count_launch();
@@ -486,7 +485,7 @@ void Bratu3D::jvp_bound32(const float* v32, double* out) {
 
 void Bratu3D::jvp_bound32f(const float* v32, float* out32) {
     if (bound_precision_ != NUMA_GPU_FP32) throw Status(NUMA_GPU_ERR_INVALID_ARGUMENT, "Bratu3D: no FP32 product bound");
-    March m = march_shape((int)n_, false);
+    March m = march_shape((int)n_, false, ctx_.sm_count);
     launch_pdl(k_jvp32f<float>, m.grid, dim3(BX, BY), 0, ctx_.stream, bound_c32_, v32, out32, (int)n_, m.ichunk,
                (float)h2inv_);
     ctx_.count_launch();
@@ -500,7 +499,7 @@ void Bratu3D::jvp_bound32x(const float* v32, double* out) {
 
 void Bratu3D::jvp_c32x(const double* c, const float* v32, double* out) {
     if (n_ >= 4095) throw Status(NUMA_GPU_ERR_NOT_SUPPORTED, "Bratu3D: the double-FP32 product needs n < 4095");
-    March m = march_shape((int)n_, false);
+    March m = march_shape((int)n_, false, ctx_.sm_count);
     launch_pdl(k_jvp32x<double>, m.grid, dim3(BX, BY), 0, ctx_.stream, c, v32, out, (int)n_, m.ichunk,
                (float)h2inv_);
     ctx_.count_launch();
@@ -509,7 +508,7 @@ void Bratu3D::jvp_c32x(const double* c, const float* v32, double* out) {
 
 void Bratu3D::jvp_bound32xf(const float* v32, float* out32) {
     if (!has_jvp32x()) throw Status(NUMA_GPU_ERR_INVALID_ARGUMENT, "Bratu3D: no FP32-input FP64-accuracy product bound");
-    March m = march_shape((int)n_, false);
+    March m = march_shape((int)n_, false, ctx_.sm_count);
     launch_pdl(k_jvp32x<float>, m.grid, dim3(BX, BY), 0, ctx_.stream, bound_c32_, v32, out32, (int)n_, m.ichunk,
                (float)h2inv_);
     ctx_.count_launch();
@@ -522,7 +521,7 @@ void Bratu3D::jvp_bound(const double* v, double* out) {
 }
 
 void Bratu3D::eval(const double* x, double* out, double* c_out, double* norm_out) {
-    const March m = march_shape((int)n_, norm_out != nullptr);
+    const March m = march_shape((int)n_, norm_out != nullptr, ctx_.sm_count);
     eval_launch(x, out, c_out, norm_out, m.grid, m.ichunk, 0, 0);
 }
 
@@ -598,26 +597,26 @@ void Bratu3D::eval_launch(const double* x, double* out, double* c_out, double* n
 // Pieces of the evaluation for an upload that overlaps it: the plane chunks of the fused-norm grid
 // shared out into up to kEvalPieces runs of whole chunks.
 int Bratu3D::eval_pieces() const {
-    const March m = march_shape((int)n_, true);
+    const March m = march_shape((int)n_, true, ctx_.sm_count);
     return (int)std::min<unsigned>(kEvalPieces, m.grid.z);
 }
 
 size_t Bratu3D::eval_piece_begin(int c) const {
-    const March m = march_shape((int)n_, true);
+    const March m = march_shape((int)n_, true, ctx_.sm_count);
     const int K = eval_pieces();
     const size_t plane0 = std::min<size_t>((size_t)(c * (int)m.grid.z / K) * m.ichunk, n_);
     return plane0 * n_ * n_;
 }
 
 size_t Bratu3D::eval_piece_need(int c) const {
-    const March m = march_shape((int)n_, true);
+    const March m = march_shape((int)n_, true, ctx_.sm_count);
     const int K = eval_pieces();
     const size_t plane1 = std::min<size_t>((size_t)((c + 1) * (int)m.grid.z / K) * m.ichunk, n_);
     return std::min(plane1 + 1, n_) * n_ * n_;  // its planes and the next one (the stencil's i + 1)
 }
 
 void Bratu3D::eval_piece(const double* x, double* out, double* cache, int c, double* sumsq) {
-    const March m = march_shape((int)n_, true);
+    const March m = march_shape((int)n_, true, ctx_.sm_count);
     const int K = eval_pieces();
     const int z0 = c * (int)m.grid.z / K, z1 = (c + 1) * (int)m.grid.z / K;
     eval_launch(x, out, cache, sumsq, dim3(m.grid.x, m.grid.y, (unsigned)(z1 - z0)), m.ichunk, z0, 1);
@@ -630,14 +629,14 @@ void Bratu3D::coef(const double* x, double* c) {
 }
 
 void Bratu3D::jvp_c(const double* c, const double* v, double* out) {
-    March m = march_shape((int)n_, false);
+    March m = march_shape((int)n_, false, ctx_.sm_count);
     launch_pdl(k_jvp<false>, m.grid, dim3(BX, BY), 0, ctx_.stream, c, v, out, (int)n_, m.ichunk, lambda_, h2inv_);
     ctx_.count_launch();
     ctx_.check_launch("bratu3d jvp");
 }
 
 void Bratu3D::jvp_c32(const float* c32, const double* v, double* out) {
-    March m = march_shape((int)n_, false);
+    March m = march_shape((int)n_, false, ctx_.sm_count);
     launch_pdl(k_jvp32<double>, m.grid, dim3(BX, BY), 0, ctx_.stream, c32, v, out, (int)n_, m.ichunk, (float)h2inv_);
     ctx_.count_launch();
     ctx_.check_launch("bratu3d jvp32");
@@ -646,7 +645,7 @@ void Bratu3D::jvp_c32(const float* c32, const double* v, double* out) {
 // The FP32 Jacobian product of Bratu3D(n) with a given FP32 coefficient, and RN32(c), for callers
 // that hold the coefficient themselves (the learned preconditioner).
 void bratu_jvp32(Context& ctx, int n, double h2inv, const float* c32, const double* v, double* out) {
-    March m = march_shape(n, false);
+    March m = march_shape(n, false, ctx.sm_count);
     launch_pdl(k_jvp32<double>, m.grid, dim3(BX, BY), 0, ctx.stream, c32, v, out, n, m.ichunk, (float)h2inv);
     ctx.count_launch();
     ctx.check_launch("bratu jvp32");
@@ -664,7 +663,7 @@ void Bratu3D::coef32(const double* c, float* c32) {
 }
 
 void Bratu3D::jvp_x(const double* x, const double* v, double* out) {
-    March m = march_shape((int)n_, false);
+    March m = march_shape((int)n_, false, ctx_.sm_count);
     launch_pdl(k_jvp<true>, m.grid, dim3(BX, BY), 0, ctx_.stream, x, v, out, (int)n_, m.ichunk, lambda_, h2inv_);
     ctx_.count_launch();
     ctx_.check_launch("bratu3d jvp(x)");

@@ -210,8 +210,7 @@ __global__ void __launch_bounds__(256) k_b2_eval(const double* __restrict__ w, c
         }
     }
     if (NORM) {
-        __shared__ double sm[1][32];
-        block_sum<1>(acc, sm);
+        block_sum<1>(acc);
         grid_reduce_finish<1>(acc, red, [norm_out] __device__(const double(&t)[1]) { *norm_out = __dsqrt_rn(t[0]); }, host);
     }
 }
@@ -1248,6 +1247,7 @@ __global__ void k_bmg_out(const T* __restrict__ X, int n, double* __restrict__ z
 constexpr int kBmgCoarsestSweeps = 30;
 constexpr int kBmgOneBlockPoints = 4096;
 constexpr int kBmgTailMaxN = 64;  // levels this small (below the finest; half in FP64) run in the one-block tail
+static_assert((4 << (kBmgTailLevels - 1)) >= kBmgTailMaxN, "a tail halves down to 4 points a side");
 
 }  // namespace
 

@@ -99,16 +99,18 @@ __device__ __forceinline__ void warp_sum_scatter(double (&v)[R]) {
     for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
 }
 
-// Block-wide sum of R <= 8 values per thread; every thread of the block (at most 256) must call it.  Returns the
-// block totals in warp 0 lane 0 (others hold unspecified values).  One butterfly a warp and value, as it was, is 5
+// Block-wide sum of R <= 8 values per thread; every thread of the block must call it, of a kernel whose launch bounds
+// hold it to kRedThreads threads.  Returns the block totals in warp 0 lane 0 (others hold unspecified values).  One butterfly a warp and value, as it was, is 5
 // FP64 additions on each of eight warps; one value is instead summed from shared memory by warp 0 (12 in all), several
 // by warp_sum_scatter.
 template <int R>
-__device__ __forceinline__ void block_sum(double (&v)[R], double (*smem)[32]) {
+__device__ __forceinline__ void block_sum(double (&v)[R]) {
+    static_assert(R >= 1 && R <= 8, "one warp sums eight results at most");
+    static_assert(kRedThreads == 256, "eight warps: the sums below take one value of each");
     const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
     const int nthreads = blockDim.x * blockDim.y * blockDim.z;
     if constexpr (R == 1) {
-        __shared__ double buf[256];
+        __shared__ double buf[kRedThreads];
         buf[tid] = v[0];
         __syncthreads();
         if (tid < 32) {
@@ -117,8 +119,8 @@ __device__ __forceinline__ void block_sum(double (&v)[R], double (*smem)[32]) {
             for (int k = 0; k < 8; ++k) t[k] = tid + 32 * k < nthreads ? buf[tid + 32 * k] : 0.0;
             v[0] = warp_sum(((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7])));
         }
-        (void)smem;
     } else {
+        __shared__ double smem[R][kRedThreads / 32];
         constexpr int RP = R <= 2 ? 2 : (R <= 4 ? 4 : 8), SH = RP == 2 ? 4 : (RP == 4 ? 3 : 2);  // lane >> SH: result
         const int lane = tid & 31, warp = tid >> 5, nwarps = (nthreads + 31) >> 5;
         double p[RP];
@@ -152,7 +154,6 @@ __device__ __forceinline__ void block_sum(double (&v)[R], double (*smem)[32]) {
 template <int R, class Fin>
 __device__ __forceinline__ void grid_reduce_finish(const double (&v)[R], RedArgs red, Fin fin, HostOut host = {}) {
     __shared__ bool am_last;
-    __shared__ double tot_smem[R][32];
     const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
     const unsigned nblocks = gridDim.x * gridDim.y * gridDim.z;
     const unsigned bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
@@ -174,7 +175,7 @@ __device__ __forceinline__ void grid_reduce_finish(const double (&v)[R], RedArgs
         for (unsigned b = tid; b < nblocks; b += nthreads) s += __ldcg(red.partials + (size_t)r * kMaxRedBlocks + b);
         acc[r] = s;
     }
-    block_sum<R>(acc, tot_smem);
+    block_sum<R>(acc);
     if (tid == 0) {
         fin(acc);
         *red.ticket = 0u;

@@ -150,12 +150,11 @@ __global__ void __launch_bounds__(kRedThreads) k_dot(const double* __restrict__ 
                                                      size_t N, RedArgs red, Fin fin, HostOut host) {
     pdl_wait();
     pdl_trigger();
-    __shared__ double sm[1][32];
     double s[1] = {0.0};
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += stride)
         s[0] = __fma_rn(a[i], b[i], s[0]);
-    block_sum<1>(s, sm);
+    block_sum<1>(s);
     grid_reduce_finish<1>(s, red, fin, host);
 }
 

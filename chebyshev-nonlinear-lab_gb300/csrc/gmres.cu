@@ -64,7 +64,6 @@ __global__ void __launch_bounds__(kRedThreads) k_mgs(double* __restrict__ w, con
                                                      HostOut host = {}) {
     pdl_wait();
     pdl_trigger();
-    __shared__ double sm[1][32];
     double s[1] = {0.0};
     const double a = HAS_PREV ? -(*hprev) : 0.0;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -76,7 +75,7 @@ __global__ void __launch_bounds__(kRedThreads) k_mgs(double* __restrict__ w, con
         }
         s[0] = NORM ? __fma_rn(wi, wi, s[0]) : __fma_rn(wi, Vcur[i], s[0]);
     }
-    block_sum<1>(s, sm);
+    block_sum<1>(s);
     grid_reduce_finish<1>(s, red, fin, host);
 }
 
@@ -197,7 +196,6 @@ __global__ void __launch_bounds__(kRedThreads) k_icwy_update(double* __restrict_
     pdl_wait();
     pdl_trigger();
     __shared__ double h[kIcwyMax];
-    __shared__ double sm[1][32];
     if (threadIdx.x < kIcwyMax) h[threadIdx.x] = threadIdx.x <= j ? hcol[threadIdx.x] : 0.0;
     __syncthreads();
     double s[1] = {0.0};
@@ -217,7 +215,7 @@ __global__ void __launch_bounds__(kRedThreads) k_icwy_update(double* __restrict_
         w[i] = wi;
         s[0] = __fma_rn(wi, wi, s[0]);
     }
-    block_sum<1>(s, sm);
+    block_sum<1>(s);
     grid_reduce_finish<1>(s, red, fin, host);
 }
 
@@ -264,7 +262,6 @@ __global__ void __launch_bounds__(kRedThreads) k_cgs(const double* w, const doub
     pdl_wait();
     pdl_trigger();
     constexpr int R = MODE == 2 ? 1 : CNT;
-    __shared__ double sm[R][32];
     double hs[CNT];
 #pragma unroll
     for (int r = 0; r < CNT; ++r) hs[r] = MODE != 0 ? hin[r] * (sig2 ? sig2[r] : 1.0) : 0.0;
@@ -287,7 +284,7 @@ __global__ void __launch_bounds__(kRedThreads) k_cgs(const double* w, const doub
         }
     }
     if constexpr (MODE != 3) {
-        block_sum<R>(s, sm);
+        block_sum<R>(s);
         grid_reduce_finish<R>(s, red, [hout, sig2_out] __device__(const double(&t)[R]) {
             if (MODE == 2) {
                 const double nrm = __dsqrt_rn(t[0]);
@@ -455,7 +452,6 @@ __global__ void __launch_bounds__(kRedThreads) k_cgs_df(const float* w, const fl
     pdl_wait();
     pdl_trigger();
     constexpr int R = MODE == 2 ? 1 : CNT;
-    __shared__ double sm[R][32];
     DF cw{0.0f, 0.0f}, c[CNT];
     if (MODE != 0) {
         const double a = ascale ? *ascale : 1.0;
@@ -521,7 +517,7 @@ __global__ void __launch_bounds__(kRedThreads) k_cgs_df(const float* w, const fl
         double s[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) s[r] = df_to_f64(acc[r]);
-        block_sum<R>(s, sm);
+        block_sum<R>(s);
         grid_reduce_finish<R>(s, red, [hout, sig2, sig, j] __device__(const double(&t)[R]) {
             if (MODE == 2) {
                 const double nrm = __dsqrt_rn(t[0]);

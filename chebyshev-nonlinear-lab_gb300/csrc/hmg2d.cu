@@ -305,6 +305,9 @@ __global__ void __launch_bounds__(1024) k_htile_up(const double* __restrict__ b,
     }
 }
 
+static_assert(kTailTop * ((kTailTop + 1) / 2) <= kTailThreads && (kTailTop / 2) * (kTailTop / 2) <= kTailThreads,
+              "htail_sweeps and htail_restrict: a thread for each pair, and for each coarse point");
+
 // x at padded index P
 __device__ __forceinline__ double& hx(double* X, int H, int P) { return X[(P & 1) * H + (P >> 1)]; }
 
@@ -313,7 +316,7 @@ __device__ __noinline__ void htail_sweeps(const HTailLvl& T, int sweeps, int ord
     const int n = L.n, m = T.m, H = T.H, np = (n + 1) >> 1;
     double* X = htail_smem + T.offX;
     const double* B = htail_smem + T.offB;
-    const int i = (int)threadIdx.x / np, j0 = 2 * ((int)threadIdx.x - i * np);  // n np <= kTailThreads
+    const int i = (int)threadIdx.x / np, j0 = 2 * ((int)threadIdx.x - i * np);
 #pragma unroll 1
     for (int p = 0; p < 2 * sweeps; ++p) {
         const int colour = (p & 1) ^ (alternate ? (p >> 1) & 1 : order);
@@ -355,7 +358,7 @@ __device__ __noinline__ void htail_residual(const HTailLvl& T, double* R) {
 
 __device__ __noinline__ void htail_restrict(const double* R, int nf, double* B, int nc) {
     const double w[3] = {0.25, 0.5, 0.25};
-    const int t = threadIdx.x;  // nc <= 15
+    const int t = threadIdx.x;
     if (t < nc * nc) {
         const int I = t / nc, J = t - I * nc;
         const double* row = R + 2 * I * nf + 2 * J;

@@ -212,8 +212,7 @@ __global__ void __launch_bounds__(256) k_bias_grad(const uint4* __restrict__ g, 
         s += f[q];
     }
     double acc[1] = {(double)s};
-    __shared__ double sm[1][32];
-    block_sum<1>(acc, sm);
+    block_sum<1>(acc);
     if (threadIdx.x == 0) db[co] += (float)acc[0];
 }
 

@@ -45,6 +45,7 @@ constexpr int kCoarseMax = 8;  // levels of one launch
 constexpr int kCoarseTop = 15, kCoarseSolo = 7;
 constexpr int kCoarseCluster = 8;
 constexpr int kCoarseThreads = 512;
+static_assert(kCoarseTop * ((kCoarseTop + 1) / 2) <= kCoarseThreads, "a thread for each pair of a plane");
 
 struct CoarseLvl {
     int n, m, pl, owners;  // pitch, planes a CTA, CTAs that own planes
@@ -469,7 +470,7 @@ inline size_t coarse_layout(CoarseParams& cp, const int* n, const double* h2inv,
         L.owners = (n[l] + L.pl - 1) / L.pl;
         L.H = ((L.pl + 2) * L.m * L.m + 2) / 2;
         L.cols = n[l] * ((n[l] + 1) / 2);
-        L.G = kCoarseThreads / L.cols;  // (>= 1: the sizes the coarse kernel takes have at most 496 columns)
+        L.G = kCoarseThreads / L.cols;
         L.mnp = magic_div((n[l] + 1) / 2);
         L.mn = magic_div(n[l]);
         L.mcols = magic_div(L.cols);

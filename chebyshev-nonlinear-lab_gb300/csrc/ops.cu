@@ -14,11 +14,10 @@ namespace {
 // direction raises the flag that makes the quotient kernels write zeros (operator.hpp:105-106).
 __global__ void __launch_bounds__(kRedThreads) k_fd_step(const double* __restrict__ v, size_t N, RedArgs red,
                                                          double scale, double* slots /* h, h^2, zero, xnorm, RN(1/h), RN(1/h^2) */) {
-    __shared__ double sm[1][32];
     double s[1] = {0.0};
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += stride) s[0] = __fma_rn(v[i], v[i], s[0]);
-    block_sum<1>(s, sm);
+    block_sum<1>(s);
     grid_reduce_finish<1>(s, red, [slots, scale] __device__(const double(&t)[1]) {
         const double nv = __dsqrt_rn(t[0]);
         if (nv == 0.0) {
@@ -117,8 +116,7 @@ __global__ void __launch_bounds__(256) k_burgers_eval(const double* __restrict__
         if (NORM) acc[0] = __fma_rn(fv, fv, __fma_rn(fu, fu, acc[0]));
     }
     if (NORM) {
-        __shared__ double sm[1][32];
-        block_sum<1>(acc, sm);
+        block_sum<1>(acc);
         grid_reduce_finish<1>(acc, red, [norm_out] __device__(const double(&t)[1]) { *norm_out = __dsqrt_rn(t[0]); }, host);
     }
 }
