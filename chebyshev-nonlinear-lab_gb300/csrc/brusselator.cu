@@ -1113,16 +1113,13 @@ __global__ void __launch_bounds__(kBmgTailThreads<T>, 1) k_bmg_tail(const TailLv
     };
     auto coarsest = [&]() {
         const int kc = count - 1, n = desc[kc].n;
-        const bool small = kc >= kw;
-        const int tid = threadIdx.x, nt = small ? 32 : blockDim.x;
         T* X = base + desc[kc].off;
-        if (small) {  // n <= 8: a lane has one point of each colour
+        if (kc >= kw) {  // n <= 8, warp 0: a lane has one point of each colour
             tail_coarsest_warp(X, n, tail_args<T>(desc[kc]), sweeps);
             return;
         }
-        for (int q = tid; q < 2 * n * n; q += nt) X[q] = T(0);
-        if (small) __syncwarp();
-        else __syncthreads();
+        for (int q = threadIdx.x; q < 2 * n * n; q += blockDim.x) X[q] = T(0);
+        __syncthreads();
         for (int s = 0; s < sweeps; ++s) {
             pass(kc, 0, false);
             pass(kc, 1, false);

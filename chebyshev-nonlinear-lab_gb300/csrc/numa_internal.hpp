@@ -388,8 +388,6 @@ public:
     // Diagnostic: average time (ms) of one red-black colour pass on the finest level, timed with
     // CUDA events over `reps` back-to-back passes on the context stream.
     double time_finest_pass(int reps);
-    // FP32 cycle: RN32(r) of the last apply on the finest level and its layout (colour-split when odd).
-    const float* fine_b32() const;
     // Jacobian-aware coarse levels (FP32 cycle with a one-CTA tail): the levels n <= 15 then solve
     // with -Lap_h - c instead of -Lap_h, c the full-weighting restriction of the fine coefficient c
     // (for Bratu3D's Jacobian, c = lambda e^u) set by set_coarse_coefficient.

@@ -79,17 +79,6 @@ PoissonMG::PoissonMG(Context& ctx, size_t n, int pre, int post, int precision, i
         L->n = static_cast<int>(m);
         L->h2inv = h2;
         L->inv = 1.0 / h2;
-        const size_t Nl = m * m * m;
-        if (precision == NUMA_GPU_FP32) {
-            // x is padded by more than one plane of a colour on both sides, b and b h^2 at the end:
-            // the FP32 kernels load every neighbour unconditionally (boundary values are then
-            // replaced by zero with a select), and no load leaves the allocation
-            const size_t pad = ((m * m - 1) / 2 + m + 2 + 31) / 32 * 32;
-            L->x32.resize(Nl + 2 * pad);
-            L->xs = L->x32.p + pad;
-            L->b32.resize(Nl + 64);
-            L->bs32.resize(Nl + 64);
-        }
         levels_.push_back(std::move(L));
         if (m % 2 == 0 || m <= 1) break;
         if (max_levels > 0 && (int)levels_.size() >= max_levels) break;
@@ -97,22 +86,28 @@ PoissonMG::PoissonMG(Context& ctx, size_t n, int pre, int post, int precision, i
         h2 /= 4.0;
     }
     plan_chain();
-    if (precision == NUMA_GPU_FP64) {
-        if (cl_l_ == SIZE_MAX) plan_coarse();
-        for (size_t l = 0; l < levels_.size() && l <= cl_l_; ++l) {  // below, the levels live in shared memory
-            Level& L = *levels_[l];
-            const size_t Nl = (size_t)L.n * L.n * L.n;
+    if (precision == NUMA_GPU_FP64 && cl_l_ == SIZE_MAX) plan_coarse();
+    for (size_t l = 0; l < levels_.size() && l <= cl_l_; ++l) {  // below, the levels live in shared memory
+        Level& L = *levels_[l];
+        const size_t n1 = L.n, Nl = n1 * n1 * n1;
+        if (precision == NUMA_GPU_FP64) {
             L.bs64.resize(Nl);
             if (l > 0) {
                 L.x64.resize(Nl);
                 L.b64.resize(Nl);
             }
+        } else {
+            // x is padded by more than one plane of a colour on both sides, b and b h^2 at the end:
+            // the FP32 kernels load every neighbour unconditionally (boundary values are then
+            // replaced by zero with a select), and no load leaves the allocation
+            const size_t pad = ((n1 * n1 - 1) / 2 + n1 + 2 + 31) / 32 * 32;
+            L.x32.resize(Nl + 2 * pad);
+            L.xs = L.x32.p + pad;
+            L.b32.resize(Nl + 64);
+            L.bs32.resize(Nl + 64);
         }
     }
-    if (levels_.size() > 1) {
-        if (precision == NUMA_GPU_FP64) scratch_r_.resize(cl_l_ > 0 ? N0_ : 0);
-        else scratch_r_.resize((N0_ + 1) / 2);  // N0 floats
-    }
+    if (levels_.size() > 1 && cl_l_ > 0) scratch_r_.resize(precision == NUMA_GPU_FP64 ? N0_ : (N0_ + 1) / 2);  // N0 values
     // FP32: the levels of n <= 15 below the finest run as one CTA with shared-memory arrays
     if (precision == NUMA_GPU_FP32) {
         for (size_t l = 1; l < levels_.size(); ++l) {
@@ -668,8 +663,6 @@ void PoissonMG::apply(const double* r, double* z) {
     }
     ctx_.check_launch("mg apply");
 }
-
-const float* PoissonMG::fine_b32() const { return levels_[0]->b32.p; }
 
 namespace {
 
