@@ -63,7 +63,10 @@ typedef enum numa_gpu_deriv_mode {
 
 /* Arnoldi orthogonalisation. */
 typedef enum numa_gpu_orth {
-    NUMA_GPU_ORTH_MGS = 0, /* modified Gram-Schmidt, the reference (linalg/gmres.hpp:141-144) */
+    NUMA_GPU_ORTH_MGS = 0, /* modified Gram-Schmidt, the reference's (linalg/gmres.hpp:141-144): its chain of inner
+                              products and updates; from the fifth vector of a cycle to the 32nd, on vectors of at
+                              most 2^20 points, its inverse compact WY form (the same coefficients and the same
+                              kind of loss of orthogonality up to rounding, two reductions a step) */
     NUMA_GPU_ORTH_CGS2 = 1, /* classical Gram-Schmidt with one reorthogonalisation, fused multi-dot */
     NUMA_GPU_ORTH_CGS1 = 2  /* classical Gram-Schmidt, one pass (multi-dot, then update and norm) */
 } numa_gpu_orth;
