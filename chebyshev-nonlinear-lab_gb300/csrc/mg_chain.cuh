@@ -396,6 +396,14 @@ __device__ __forceinline__ void chain_coef(const float* c) {
     }
 }
 
+// b / 24: (b / 6) / 4 has one rounding where div6 is exact and the quarter does not underflow.
+__device__ __forceinline__ float chain_div24(float b) {
+    return fabsf(b) >= 0x1p-100f && fabsf(b) <= 0x1p127f ? div6(b) * 0.25f : b / 24.0f;
+}
+__device__ __forceinline__ double chain_div24(double b) {
+    return fabs(b) >= 0x1p-960 && fabs(b) <= 0x1p1023 ? div6(b) * 0.25 : b / 24.0;
+}
+
 // The levels CTA 0 holds below level A (which it has restricted): 7^3 on its warps, 3^3 and the point on warp 0.
 template <class L7, class L3, class L1, int OR>
 __device__ __forceinline__ void chain_tail(const ChainIo& io, const float* c1) {
@@ -409,8 +417,9 @@ __device__ __forceinline__ void chain_tail(const ChainIo& io, const float* c1) {
         if (threadIdx.x == 0) {
             constexpr int q = L1::H + ((13 - 1) >> 1);  // the point's padded index is 13: parity 1
             const T b = chain_base<T>()[L1::OB + q];
-            T v = div6(b) * T(0.25);  // b / 24 with one rounding
+            T v;
             if constexpr (L7::SHIFT) v = b / (T(24) - *c1);
+            else v = chain_div24(b);
             chain_base<T>()[L1::OX + q] = v;
         }
         __syncwarp();

@@ -407,9 +407,8 @@ __device__ __forceinline__ void coarse_cycle(const double* b_in, double* x_out) 
         const CoarseLvl& C = cp.L[last];
         if (C.n == 1) {
             if (threadIdx.x == 0) {
-                // x = b / (6 h^-2); n = 1 has h^-2 = 4, so b / 24 = (b / 6) / 4 with one rounding
                 const int P = (C.m + 1) * C.m + 1;
-                base[C.offX + (P & 1) * C.H + (P >> 1)] = div6(base[C.offB]) * C.inv;
+                base[C.offX + (P & 1) * C.H + (P >> 1)] = base[C.offB] / (6.0 * C.h2inv);
             }
             __syncthreads();
         } else if (C.n == 2) {

@@ -1,6 +1,6 @@
-"""The Jacobian-aware FP32 V-cycle (levels n <= 15 of -Lap_h - c) bit for bit a float32 restatement: right-hand sides of
-ordinary size, and of a size whose quotients leave the range in which a correction by the reciprocal is exact (the
-levels then divide)."""
+"""The FP32 V-cycle through the chain of coarse levels, Poisson's and the Jacobian-aware one (levels n <= 15 of
+-Lap_h - c), bit for bit a float32 restatement: right-hand sides of ordinary size, and of a size whose quotients leave
+the range in which a correction by the reciprocal is exact (the Jacobian-aware levels and the last point then divide)."""
 import numpy as np
 import pytest
 
@@ -43,7 +43,9 @@ def _interp(x):
 
 
 def vcycle32_jacobian(r, n, c, pre, post):
-    coef, m = [c.reshape(n, n, n).astype(F)], n
+    """c None: no level is shifted."""
+    poisson = c is None
+    coef, m = [np.zeros((n,) * 3, F) if poisson else c.reshape(n, n, n).astype(F)], n
     while m > 1:
         m = (m - 1) // 2
         coef.append(_weight(coef[-1], m))
@@ -51,7 +53,7 @@ def vcycle32_jacobian(r, n, c, pre, post):
     def cycle(l, b):
         m = coef[l].shape[0]
         h2 = (m + 1.0) ** 2
-        shift = l > 0 and m <= 15
+        shift = not poisson and l > 0 and m <= 15
         if m == 1:
             return b / (F(6 * h2) - coef[l])
         cs, bs, mask = coef[l] * F(1 / h2), b * F(1 / h2), colour_mask(m)
@@ -99,3 +101,13 @@ def test_jacobian_vcycle_bit_exact(gpu, n, pre, post, size):
     z = gpu.vec(n ** 3)
     pc.apply(gpu.from_numpy(r), z)
     assert np.array_equal(z.numpy(), vcycle32_jacobian(r, n, 6.0 * 2.0 ** k, pre, post))
+
+
+@pytest.mark.parametrize("n,pre,post", [(31, 2, 2), (63, 1, 2)])
+@pytest.mark.parametrize("size", [1.0, 1e-37])
+def test_poisson_vcycle_bit_exact(gpu, n, pre, post, size):
+    import numa_gpu as G
+    r = size * np.random.default_rng(n).standard_normal(n ** 3)
+    mg, z = G.PoissonMG(gpu, n, pre, post, precision=G.FP32), gpu.vec(n ** 3)
+    mg(gpu.from_numpy(r), z)
+    assert np.array_equal(z.numpy(), vcycle32_jacobian(r, n, None, pre, post))
