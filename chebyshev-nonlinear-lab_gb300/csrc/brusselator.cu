@@ -1022,17 +1022,15 @@ __global__ void __launch_bounds__(kBmgTailThreads<T>, 1) k_bmg_tail(const TailLv
             break;
         }
     const bool warp0 = threadIdx.x < 32;
-    // one colour pass of level k by threads [0, nt); then the barrier of that group
-    auto pass = [&](int k, int colour, bool first) {
-        const bool small = k >= kw;
+    // one colour pass of level L (a copy in registers: from shared memory its constants would be loaded again behind
+    // every barrier) by the block, or by warp 0 (small); then the barrier of that group
+    auto pass = [&](const TailLvl& L, bool small, int colour, bool first) {
         const int tid = threadIdx.x, nt = small ? 32 : blockDim.x;
-        const TailLvl L = desc[k];
         const int n = L.n, half = n / 2;
         T* X = base + L.off;
         const T* Bv = X + 2 * n * n;
         const T* K = X + 4 * n * n;
         const LvlArgs<T>& A = tail_args<T>(L);
-        const T su = A.su, sv = A.sv, su4 = A.su4, sv4 = A.sv4;
         for (int idx = tid; idx < n * half; idx += nt) {
             const int i = idx / half, jj = idx - i * half;
             const int j = 2 * jj + ((i + colour) & 1);
@@ -1040,7 +1038,7 @@ __global__ void __launch_bounds__(kBmgTailThreads<T>, 1) k_bmg_tail(const TailLv
             const auto b = ld2(Bv, p);
             T Su = T(0), Sv = T(0), u, v;
             if (!first) nbr_sums(X, n, i, j, Su, Sv);
-            block_update(load_blk_s(K, p), su, sv, su4, sv4, b.x, b.y, Su, Sv, u, v);
+            block_update(load_blk_s(K, p), A.su, A.sv, A.su4, A.sv4, b.x, b.y, Su, Sv, u, v);
             st2(X, p, u, v);
         }
         if (small) __syncwarp();
@@ -1096,19 +1094,23 @@ __global__ void __launch_bounds__(kBmgTailThreads<T>, 1) k_bmg_tail(const TailLv
         else __syncthreads();
     };
     auto down = [&](int k) {
-        pass(k, 0, true);
-        pass(k, 1, false);
+        const TailLvl L = desc[k];
+        const bool small = k >= kw;
+        pass(L, small, 0, true);
+        pass(L, small, 1, false);
         for (int s = 1; s < pre; ++s) {
-            pass(k, 0, false);
-            pass(k, 1, false);
+            pass(L, small, 0, false);
+            pass(L, small, 1, false);
         }
         restrict_to(k);
     };
     auto up = [&](int k) {
         prolong_from(k);
+        const TailLvl L = desc[k];
+        const bool small = k >= kw;
         for (int s = 0; s < post; ++s) {
-            pass(k, 1, false);
-            pass(k, 0, false);
+            pass(L, small, 1, false);
+            pass(L, small, 0, false);
         }
     };
     auto coarsest = [&]() {
@@ -1120,9 +1122,10 @@ __global__ void __launch_bounds__(kBmgTailThreads<T>, 1) k_bmg_tail(const TailLv
         }
         for (int q = threadIdx.x; q < 2 * n * n; q += blockDim.x) X[q] = T(0);
         __syncthreads();
+        const TailLvl L = desc[kc];
         for (int s = 0; s < sweeps; ++s) {
-            pass(kc, 0, false);
-            pass(kc, 1, false);
+            pass(L, false, 0, false);
+            pass(L, false, 1, false);
         }
     };
     {
