@@ -29,10 +29,19 @@ struct March {
 // more when it would exceed kMaxRedBlocks partials.  Smaller grids halve the chunk until there are four
 // blocks an SM: a march of 4 planes at 31^3 left four SMs in five idle and was bound by the latency of
 // its FP64 operations (the product from x 5.8 us, with one plane a thread 2.8; with c given 4.5 and 2.5).
-March march_shape(int n, bool reducing, int sm_count) {
+// A reduction, whose every block costs half a plane more, also stops at one to two blocks an SM, which all run at once:
+// between two and four an SM the evaluation takes as long as four would (88^3 in chunks of 8 35.0 us, of 4
+// 24.1), and past that its blocks add up (63^3, FP64 and mixed: chunks of 4 12.2 and 10.7 us, of 1, for
+// four blocks an SM, 14.0 and 12.5; 80^3 in chunks of 8 20.5 and 16.7, of 2 22.1 and 17.9).  Not where the grid is
+// launched in pieces: a piece has an eighth of its blocks, and the latency of its chunk bounds it.
+March march_shape(int n, bool reducing, int sm_count, bool pieces = false) {
     const int kb = (n + BX - 1) / BX, jb = (n + BY - 1) / BY;
     int ichunk = reducing && n >= 128 ? 16 : 8;
-    while (ichunk > 1 && (long)kb * jb * ((n + ichunk - 1) / ichunk) < 4L * sm_count) ichunk /= 2;
+    for (; ichunk > 1; ichunk /= 2) {
+        const long blocks = (long)kb * jb * ((n + ichunk - 1) / ichunk);
+        if (blocks >= 4L * sm_count) break;
+        if (reducing && !pieces && 10 * blocks >= 9L * sm_count && blocks <= 2L * sm_count) break;
+    }
     if (reducing) {
         const long cols = (long)kb * jb;
         const long max_chunks = kMaxRedBlocks / cols;
@@ -597,26 +606,26 @@ void Bratu3D::eval_launch(const double* x, double* out, double* c_out, double* n
 // Pieces of the evaluation for an upload that overlaps it: the plane chunks of the fused-norm grid
 // shared out into up to kEvalPieces runs of whole chunks.
 int Bratu3D::eval_pieces() const {
-    const March m = march_shape((int)n_, true, ctx_.sm_count);
+    const March m = march_shape((int)n_, true, ctx_.sm_count, true);
     return (int)std::min<unsigned>(kEvalPieces, m.grid.z);
 }
 
 size_t Bratu3D::eval_piece_begin(int c) const {
-    const March m = march_shape((int)n_, true, ctx_.sm_count);
+    const March m = march_shape((int)n_, true, ctx_.sm_count, true);
     const int K = eval_pieces();
     const size_t plane0 = std::min<size_t>((size_t)(c * (int)m.grid.z / K) * m.ichunk, n_);
     return plane0 * n_ * n_;
 }
 
 size_t Bratu3D::eval_piece_need(int c) const {
-    const March m = march_shape((int)n_, true, ctx_.sm_count);
+    const March m = march_shape((int)n_, true, ctx_.sm_count, true);
     const int K = eval_pieces();
     const size_t plane1 = std::min<size_t>((size_t)((c + 1) * (int)m.grid.z / K) * m.ichunk, n_);
     return std::min(plane1 + 1, n_) * n_ * n_;  // its planes and the next one (the stencil's i + 1)
 }
 
 void Bratu3D::eval_piece(const double* x, double* out, double* cache, int c, double* sumsq) {
-    const March m = march_shape((int)n_, true, ctx_.sm_count);
+    const March m = march_shape((int)n_, true, ctx_.sm_count, true);
     const int K = eval_pieces();
     const int z0 = c * (int)m.grid.z / K, z1 = (c + 1) * (int)m.grid.z / K;
     eval_launch(x, out, cache, sumsq, dim3(m.grid.x, m.grid.y, (unsigned)(z1 - z0)), m.ichunk, z0, 1);
