@@ -353,7 +353,7 @@ struct BatchSolver::Impl {
             return MgPool{x.p + pad, b.p, bs.p, r.p, N + 2 * pad, N + 64, N, inst.p};
         }
     };
-    std::vector<std::unique_ptr<Pool>> pools;  // sizes n_max ... 15 (the last one is the tail)
+    std::vector<std::unique_ptr<Pool>> pools;  // sizes n_max ... 15 (the last two are the chain's)
     using ChainKernel = void (*)(MgPool, const int*, int, const float*, float*, ChainIo);
     ChainKernel chain_kern = nullptr;
     size_t chain_smem = 0;
@@ -436,7 +436,7 @@ struct BatchSolver::Impl {
 namespace {
 
 bool batch_size_ok(size_t n) {
-    // 2^k - 1 with k >= 5: odd down to the tail at 15 and an FP32 output on the finest level
+    // 2^k - 1 with k >= 5: the levels from 31^3 down are the chain kernel's
     if (n < 31 || n > 1023) return false;
     return ((n + 1) & n) == 0;
 }
@@ -452,8 +452,8 @@ BatchSolver::BatchSolver(Context& ctx, const numa_batch_instance* inst, size_t c
     for (size_t i = 0; i < count; ++i)
         if (!batch_size_ok(inst[i].n))
             throw Status(NUMA_GPU_ERR_NOT_SUPPORTED,
-                         "batched solver: grid sizes must be 2^k - 1 between 31 and 1023 (the FP32 multigrid "
-                         "hierarchy ends in the one-CTA tail at 15)");
+                         "batched solver: grid sizes must be 2^k - 1 between 31 and 1023 (the FP32 multigrid's "
+                         "levels from 31 down run in one kernel)");
     M.kp = p;
     M.I = (int)count;
     M.m = (int)p.restart;

@@ -52,7 +52,7 @@ private:
 };
 
 // The FP32 V-cycle with Jacobian-aware coarse levels, bound at each iterate: make() restricts the
-// iterate's coefficient c = lambda e^x (the operator's cache) down to the one-CTA tail.
+// iterate's coefficient c = lambda e^x (the operator's cache) down to the levels n <= 15.
 class JacobianMGProvider : public Provider {
 public:
     JacobianMGProvider(Context& ctx, size_t n, int pre, int post) : mg_(ctx, n, pre, post, NUMA_GPU_FP32, 0) {

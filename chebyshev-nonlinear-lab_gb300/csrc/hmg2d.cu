@@ -21,7 +21,6 @@
 #include <cmath>
 #include <limits>
 
-
 #include "numa_internal.hpp"
 
 namespace numa::gpu {

@@ -3,9 +3,10 @@
 //
 // Why.  A launched pass over such a level costs its launch (2.2-2.6 us with programmatic dependent launch
 // inside a graph), not its work, and a level is 11 such steps (60 passes more where the hierarchy ends in an
-// even grid).  Here a step is a barrier: a V(2,2) at 7^3 takes 20 us instead of 36, at 15^3 37
-// instead of 63, at 23^3 (23, 11, 5, 2) 74 instead of 115, at 63^3 109 instead of 126.  What bounds it now is latency:
-// the eight dependent FP64 operations of a point are ~520 of a pass's ~1,000 cycles on the small levels.
+// even grid).  Here a step is a barrier: a V(2,2) at 7^3 takes 19 us instead of 37, at 11^3 (11, 5, 2) 31 instead of
+// 103, at 23^3 (23, 11, 5, 2) 54 instead of 134, at 95^3 202 instead of 259.  What bounds it now is latency: the eight
+// dependent FP64 operations of a point are ~520 of a pass's ~1,000 cycles on the small levels.  (Hierarchies of 2^k - 1
+// points down to one, from 15^3 on, take mg_chain.cuh's form with its sizes at compile time.)
 //
 // Split of the work.  FP64 runs at two operations a clock on an SM, so one SM's pass over 15^3 takes 6,700
 // cycles: the top level, where it is larger than 7 points a side, is cut into slabs of pl i-planes (an

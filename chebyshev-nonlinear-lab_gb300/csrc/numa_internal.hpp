@@ -388,7 +388,7 @@ public:
     // Diagnostic: average time (ms) of one red-black colour pass on the finest level, timed with
     // CUDA events over `reps` back-to-back passes on the context stream.
     double time_finest_pass(int reps);
-    // Jacobian-aware coarse levels (FP32 cycle with a one-CTA tail): the levels n <= 15 then solve
+    // Jacobian-aware coarse levels (FP32 cycle with levels n <= 15 below the finest): they then solve
     // with -Lap_h - c instead of -Lap_h, c the full-weighting restriction of the fine coefficient c
     // (for Bratu3D's Jacobian, c = lambda e^u) set by set_coarse_coefficient.
     bool supports_coarse_jacobian() const { return precision_ == NUMA_GPU_FP32 && tail_l_ != SIZE_MAX; }
@@ -403,7 +403,7 @@ private:
     void cycle32(size_t l);
     bool first_fused32(size_t l) const;
     bool first_fused64(size_t l) const;
-    // FP32 cycle: levels from tail_l_ (n <= 15) down run in one CTA (k_mg_tail); SIZE_MAX = none.
+    // FP32 cycle: levels from tail_l_ (n <= 15) down run in one CTA (k_mg_tail) where no chain has taken them; SIZE_MAX = none.
     size_t tail_l_ = SIZE_MAX;
     size_t tail_smem_ = 0;
     void launch_tail32();

@@ -428,12 +428,12 @@ bool PoissonMG::first_fused64(size_t l) const {
 
 // The FP32 cycle (precision extension): the same steps as cycle<double> in single precision.
 // Levels of odd n (all but an even coarsest) keep x, b and b h^2 in the colour-split layout
-// (mg_kernels.cuh), where every colour pass streams its own colour contiguously.  Three fusions
+// (mg_kernels.cuh), where every colour pass streams its own colour contiguously.  Four fusions
 // remove whole passes over the finest level: the first smoothing pass of a split level (colour 0
 // from x = 0) is written by the kernel that produces the level's right-hand side (the FP64 to
-// FP32 conversion of r, or the restriction); the last pass of the cycle writes z in FP64 for
-// both colours instead of storing x; and prolongation touches only the colour-0 fine points when
-// post-smoothing follows.
+// FP32 conversion of r, or the restriction); at 63^3, 127^3 and 255^3 the residual is restricted as it is
+// formed; the prolongation is part of the first post-smoothing pass, which alone reads the values it
+// corrects; and the last pass of the cycle writes z in FP64 for both colours instead of storing x.
 
 // True when level l's first smoothing pass is fused into the producer of its right-hand side.
 bool PoissonMG::first_fused32(size_t l) const {
@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(BX* BY) k_restrict_coef(const TI* __restrict__
 
 void PoissonMG::set_coarse_coefficient(const double* c_fine, const float* c32_fine) {
     if (!supports_coarse_jacobian())
-        throw Status(NUMA_GPU_ERR_NOT_SUPPORTED, "Jacobian-aware coarse levels need the FP32 cycle with a one-CTA tail");
+        throw Status(NUMA_GPU_ERR_NOT_SUPPORTED, "Jacobian-aware coarse levels need the FP32 cycle with levels of n <= 15 below the finest");
     if (cl_off_.empty()) {
         size_t total = 0;
         cl_off_.assign(levels_.size(), 0);

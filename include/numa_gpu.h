@@ -280,7 +280,7 @@ int numa_gpu_provider_create_poisson_mg(numa_gpu_ctx* ctx, size_t n, int pre, in
                                         numa_gpu_provider** out);
 int numa_gpu_provider_create_jacobi(numa_gpu_bratu3d* op, numa_gpu_provider** out);
 /* No counterpart in the reference (whose PoissonMGProvider, linalg/poisson_mg.hpp:303-320, ignores
- * the iterate): the FP32 PoissonMG V-cycle whose coarse levels n <= 15 (the one-CTA tail) solve with
+ * the iterate): the FP32 PoissonMG V-cycle whose coarse levels n <= 15 solve with
  * the Jacobian -Lap_h - c instead of -Lap_h, c the full-weighting restriction of the Bratu3D
  * coefficient lambda e^u of the iterate the provider is bound at (make reads the operator's cache).
  * The fine levels keep the Poisson smoother: the shift matters only for the smooth modes, which the
