@@ -212,7 +212,7 @@ void dispatch_driver(int method, NonlinearOp& f, double* x, const numa_krylov_pa
 }
 
 // out = F'(x) v or F''(x)[v, v] of any operator, analytic or by finite differences, for the
-// per-operator entry points (temporaries are freed on return, hence the synchronisation).
+// per-operator entry points (those that free temporaries on return synchronise the stream first).
 void op_derivative(NonlinearOp& f, bool second, const double* x, const double* v, double* out, int mode) {
     Context& c = f.ctx();
     const size_t N = f.size();
